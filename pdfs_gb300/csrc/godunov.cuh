@@ -43,6 +43,7 @@ struct GodConst32 {
   float q[3];
   float iqsum;
   float iso_h, iso_2h2, iso_h2;  // isotropic shortcuts
+  int tiny;  // a spacing is outside 1e-14 .. 1e14: discriminants may leave the normal floats
 };
 
 // Reference arithmetic.  The bubble sort of solveEikonal (phi3D_fsm.c:148-159)
@@ -122,13 +123,29 @@ __device__ __forceinline__ double god_fast64(double m0, double m1, double m2, co
   return u;
 }
 
+// sqrt of a discriminant of god32s.  FTZ: the flushing approximate root, which
+// has the same bits as the plain one on normal arguments and needs no scaling
+// steps around it (3 % of the 768^3 octant rounds).  A discriminant is 0 or at
+// least about 1e-8 h^2, so only spacings near the ends of the float range
+// (GodConst32::tiny) make a subnormal one: they take FTZ = false.
+template <bool FTZ>
+__device__ __forceinline__ float sqrt_disc(float x) {
+  if constexpr (FTZ) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+  } else {
+    return sqrtf(x);
+  }
+}
+
 // FP32 shifted form evaluated branch-free: all three candidates are computed
 // and the Godunov selection (1 term unless it exceeds the second minimum, 2
 // terms unless they exceed the third) picks one.  Each candidate that can be
 // selected is finite: u2 is only chosen when m1 < m0 + h (so a is finite), u3
 // only when u2 > m2 (so b is finite); infinite minima only reach candidates
 // that are not selected.
-template <bool ISO>
+template <bool ISO, bool FTZ = false>
 __device__ __forceinline__ float god32s(float m0, float m1, float m2, const GodConst32 &k) {
   if (ISO) {
     const float lo = fminf(m0, m1), hi = fmaxf(m0, m1);
@@ -138,11 +155,11 @@ __device__ __forceinline__ float god32s(float m0, float m1, float m2, const GodC
     m1 = fmaxf(lo, mid);
     const float u1 = m0 + k.iso_h;
     const float a = m1 - m0;
-    const float u2 = fmaf(0.5f, a + sqrtf(fmaxf(fmaf(-a, a, k.iso_2h2), 0.0f)), m0);
+    const float u2 = fmaf(0.5f, a + sqrt_disc<FTZ>(fmaxf(fmaf(-a, a, k.iso_2h2), 0.0f)), m0);
     const float b = m2 - m0;
     const float s = a + b;
     const float cc = fmaf(a, a, fmaf(b, b, -k.iso_h2));
-    const float u3 = fmaf(s + sqrtf(fmaxf(fmaf(s, s, -3.0f * cc), 0.0f)), 1.0f / 3.0f, m0);
+    const float u3 = fmaf(s + sqrt_disc<FTZ>(fmaxf(fmaf(s, s, -3.0f * cc), 0.0f)), 1.0f / 3.0f, m0);
     return (u1 <= m1) ? u1 : ((u2 <= m2) ? u2 : u3);
   } else {
     float h0 = k.h[0], h1 = k.h[1], h2 = k.h[2];
@@ -153,11 +170,19 @@ __device__ __forceinline__ float god32s(float m0, float m1, float m2, const GodC
     const float u1 = m0 + h0;
     const float a = m1 - m0;
     const float sq = q0 + q1;
-    const float u2 = m0 + __fdividef(fmaf(a, q1, sqrtf(fmaxf(fmaf(-a * a, q0 * q1, sq), 0.0f))), sq);
+    const float n2 = fmaf(a, q1, sqrt_disc<FTZ>(fmaxf(fmaf(-a * a, q0 * q1, sq), 0.0f)));
+    float u2;
+    if constexpr (FTZ) {  // m0 + n2 / sq as the plain form compiles: a reciprocal and one multiply-add
+      float rs;
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(sq));
+      u2 = __fmaf_rn(n2, rs, m0);
+    } else {
+      u2 = m0 + __fdividef(n2, sq);
+    }
     const float b = m2 - m0;
     const float B = fmaf(a, q1, b * q2);
     const float Cc = fmaf(a * a, q1, fmaf(b * b, q2, -1.0f));
-    const float u3 = fmaf(B + sqrtf(fmaxf(fmaf(B, B, -(q0 + q1 + q2) * Cc), 0.0f)), k.iqsum, m0);
+    const float u3 = fmaf(B + sqrt_disc<FTZ>(fmaxf(fmaf(B, B, -(q0 + q1 + q2) * Cc), 0.0f)), k.iqsum, m0);
     return (u1 <= m1) ? u1 : ((u2 <= m2) ? u2 : u3);
   }
 }
@@ -207,7 +232,7 @@ __device__ __forceinline__ double f2d_nonneg(float v) {
   return __hiloint2double((int)((de << 20) | (m >> 3)), (int)(m << 29));
 }
 
-template <bool ISO>
+template <bool ISO, bool FTZ = false>
 __device__ __forceinline__ double god_mixed64(double m0, double m1, double m2, const GodConst32 &k) {
   const long long k0 = dkey(m0), k1 = dkey(m1), k2 = dkey(m2);
   const bool b0 = k0 <= k1 && k0 <= k2, b1 = !b0 && k1 <= k2;  // which axis holds the base
@@ -217,7 +242,7 @@ __device__ __forceinline__ double god_mixed64(double m0, double m1, double m2, c
   const double pa = b0 ? m1 : m0, pb = (b0 || b1) ? m2 : m1;
   const float ea = d2f_nonneg(pa - base), eb = d2f_nonneg(pb - base);
   const float e0 = b0 ? 0.0f : ea, e1 = b0 ? ea : (b1 ? 0.0f : eb), e2 = (b0 || b1) ? eb : 0.0f;
-  return base + f2d_nonneg(god32s<ISO>(e0, e1, e2, k));
+  return base + f2d_nonneg(god32s<ISO, FTZ>(e0, e1, e2, k));
 }
 
 // ---- FP32 pairs ("double-float") --------------------------------------------------
@@ -273,7 +298,7 @@ __device__ __forceinline__ double p_add(double b, float x) {
 // 0, two infinite minima NaN, which counts as a tie), so the base and the
 // increments are the ones an exact comparison would pick, with the choice
 // no longer ahead of the subtractions on the update's dependency chain.
-template <bool ISO>
+template <bool ISO, bool FTZ = false>
 __device__ __forceinline__ double god_pair(double m0, double m1, double m2, const GodConst32 &k) {
   const float d10 = p_sub(m1, m0), d20 = p_sub(m2, m0), d21 = p_sub(m2, m1);
   const bool b0 = !(d10 < 0.0f) && !(d20 < 0.0f);  // which axis holds the base
@@ -284,7 +309,7 @@ __device__ __forceinline__ double god_pair(double m0, double m1, double m2, cons
   const float e0 = b0 ? 0.0f : (b1 ? __fsub_rn(0.0f, d10) : __fsub_rn(0.0f, d20));
   const float e1 = b0 ? d10 : (b1 ? 0.0f : __fsub_rn(0.0f, d21));
   const float e2 = b0 ? d20 : (b1 ? d21 : 0.0f);
-  const double g = p_add(base, god32s<ISO>(e0, e1, e2, k));
+  const double g = p_add(base, god32s<ISO, FTZ>(e0, e1, e2, k));
   return p_hi(base) < INFINITY ? g : base;  // no finite neighbour: the base
 }
 

@@ -67,39 +67,6 @@ struct PcGeo {
 
 __device__ __forceinline__ void compute_bar() { asm volatile("bar.sync 1, 256;\n" ::: "memory"); }
 
-__device__ __forceinline__ void st_relaxed_gpu_u64(unsigned long long *p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long *p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-// A value's 32-bit pieces, each tagged with the epoch in the upper word.
-template <class T>
-__device__ __forceinline__ void mail_put(unsigned long long *e, T v, int epoch) {
-  const unsigned long long tag = (unsigned long long)(unsigned)epoch << 32;
-  if constexpr (sizeof(T) == 4) {
-    st_relaxed_gpu_u64(e, tag | __float_as_uint(v));
-  } else {
-    st_relaxed_gpu_u64(e, tag | (unsigned)__double2loint(v));
-    st_relaxed_gpu_u64(e + 1, tag | (unsigned)__double2hiint(v));
-  }
-}
-template <class T>
-__device__ __forceinline__ bool mail_get(const unsigned long long *e, int epoch, T &v) {
-  const unsigned tag = (unsigned)epoch;
-  const unsigned long long w0 = ld_relaxed_gpu_u64(e);
-  if constexpr (sizeof(T) == 4) {
-    v = __uint_as_float((unsigned)w0);
-    return (unsigned)(w0 >> 32) == tag;
-  } else {
-    const unsigned long long w1 = ld_relaxed_gpu_u64(e + 1);
-    v = __hiloint2double((int)(unsigned)w1, (int)(unsigned)w0);
-    return (unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 32) == tag;
-  }
-}
-
 // A warp's max change -> the change word (FP32: float bits; FP64: the u64
 // key of change_u64), one atomic per warp.
 template <class T, int ARITH>
@@ -112,28 +79,6 @@ __device__ __forceinline__ void warp_change_out(T v, void *maxchg, int lane) {
     else
       atomicMax(reinterpret_cast<unsigned long long *>(maxchg), change_u64<T, ARITH>(v));
   }
-}
-
-// One idle round of a helper warp: lane 0 decides, for the whole warp, to give
-// up on the abort flag or after wait_cycles without progress.
-__device__ __forceinline__ bool helper_idle(const SweepArgs &a, int col, volatile int *s_abort, long long t_last,
-                                            unsigned &nap) {
-  int stop = 0;
-  if ((threadIdx.x & 31) == 0) {
-    if (*s_abort || *(volatile int *)(a.err + 1)) {
-      stop = 1;
-    } else if (cycles() - t_last > a.wait_cycles) {
-      raise_timeout(a, col, s_abort);
-      stop = 1;
-    }
-  }
-  if (__shfl_sync(0xffffffffu, stop, 0)) {
-    *s_abort = 1;
-    return true;
-  }
-  if (nap) __nanosleep(nap);
-  nap = min(nap + 32u, 128u);
-  return false;
 }
 
 // Batched rounds: the grid description of the current ticket, staged in
@@ -149,9 +94,6 @@ __device__ __forceinline__ const SweepArgs &pc_args(const SweepArgs &a0) {
     return pc_batch_args();
   else
     return a0;
-}
-__device__ __forceinline__ void fence_proxy_async_global() {
-  asm volatile("fence.proxy.async.global;\n" ::: "memory");
 }
 
 // BATCH: one launch runs a whole round -- the 8 orderings of every grid of a

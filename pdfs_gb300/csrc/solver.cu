@@ -666,6 +666,14 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
     c->prow = g->nz + 15;
     pmail_words = (size_t)((g->nx + 15) / 16) * ((g->ny + 15) / 16) * 2 * (size_t)c->prow * 16 * 2;
   }
+  // bricks: three faces per brick (T3Geo::MAIL words, two per FP64 value)
+  for (int k = 0; k < 2; ++k) {
+    const TileShape ts = k ? s64 : s32;
+    const int *nt = k ? c->nt64 : c->nt32;
+    if (ts.bz == 0 || o.precision == (k ? PDFS_PREC_FP32 : PDFS_PREC_FP64)) continue;
+    pmail_words = std::max(pmail_words, (size_t)nt[0] * nt[1] * nt[2] *
+                                            (size_t)(ts.bz * ts.ty + ts.bz * ts.tx + ts.tx * ts.ty) * (k ? 2 : 1));
+  }
   std::vector<std::pair<void **, size_t>> plan;
   auto want = [&](auto **p, size_t bytes) {
     if (bytes) plan.emplace_back(reinterpret_cast<void **>(p), bytes);
@@ -996,6 +1004,7 @@ void pdfs::fill_sweep_args(const pdfs_ctx *c, int which, int sn, const uint8_t *
   a.k32.iso_h = (float)g.dx;
   a.k32.iso_2h2 = (float)(2.0 * g.dx * g.dx);
   a.k32.iso_h2 = (float)(g.dx * g.dx);
+  a.k32.tiny = std::min(g.dx, std::min(g.dy, g.dz)) < 1e-14 || std::max(g.dx, std::max(g.dy, g.dz)) > 1e14;
 }
 
 static int run_sweep(pdfs_ctx *c, int which, int sn, const uint8_t *active, unsigned int *blk_chg, double *chg);

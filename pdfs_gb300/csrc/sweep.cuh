@@ -314,6 +314,12 @@ struct CapBound {
     else
       return __ldg(a.bcap64 + b);
   }
+  __device__ __forceinline__ static type lower(type x, type y) {  // the smaller of two bounds, off the FP64 pipe
+    if constexpr (sizeof(T) == 8 && ARITH == ARITH_PAIR)
+      return fminf(x, y);
+    else
+      return dkey(y) < dkey(x) ? y : x;
+  }
   // v < bound, so min(cap, v) == v for every cap of the block
   __device__ __forceinline__ static bool below(T v, type bnd) {
     if constexpr (sizeof(T) == 8 && ARITH == ARITH_PAIR)
@@ -345,6 +351,17 @@ __device__ __forceinline__ T node_change(T cv, T nv, float hmin) {
   else
     return fabs(cv - nv);
 }
+// Could node_change(cv, nv) exceed tmax?  FP32: |cv - nv| against tmax times
+// the divisor, less a margin far above the roundings of the product and of
+// the quotient; only when this says so is the division done.  NaN and infinities
+// compare false and go on to the division.
+template <class T, int ARITH>
+__device__ __forceinline__ bool change_may_exceed(T cv, T nv, float hmin, T tmax) {
+  if constexpr (sizeof(T) == 4)
+    return !(fabsf(cv - nv) < tmax * (fmaxf(nv, hmin) * (1.0f - 1e-5f)));
+  else
+    return true;
+}
 template <class T, int ARITH>
 __device__ __forceinline__ float change_f(T d) {  // as a float (per-block change words)
   if constexpr (sizeof(T) == 8 && ARITH == ARITH_PAIR)
@@ -369,53 +386,19 @@ __device__ __forceinline__ unsigned long long change_u64(T d) {  // the FP64 pha
 
 // The local solver of a kernel variant.  k64 / k32 are the compute warps'
 // register copies of the per-sweep constants.
-template <class T, int MODE, int ARITH, bool ISO>
-__device__ __forceinline__ T local_update(T m0, T m1, T m2, const GodConst64 &k64, const GodConst32 &k32);
-template <>
-__device__ __forceinline__ float local_update<float, MODE_MIN, ARITH_FAST, true>(float m0, float m1, float m2,
-                                                                                  const GodConst64 &,
-                                                                                  const GodConst32 &k32) {
-  return god32s<true>(m0, m1, m2, k32);
+template <class T, int MODE, int ARITH, bool ISO, bool FTZ = false>
+__device__ __forceinline__ T local_update(T m0, T m1, T m2, const GodConst64 &k64, const GodConst32 &k32) {
+  if constexpr (sizeof(T) == 4)
+    return god32s<ISO, FTZ>(m0, m1, m2, k32);
+  else if constexpr (ARITH == ARITH_REF)
+    return god_ref64(m0, m1, m2, k64);
+  else if constexpr (ARITH == ARITH_FAST)
+    return god_fast64(m0, m1, m2, k64);
+  else if constexpr (ARITH == ARITH_MIXED)
+    return god_mixed64<ISO, FTZ>(m0, m1, m2, k32);
+  else
+    return god_pair<ISO, FTZ>(m0, m1, m2, k32);
 }
-template <>
-__device__ __forceinline__ float local_update<float, MODE_MIN, ARITH_FAST, false>(float m0, float m1, float m2,
-                                                                                   const GodConst64 &,
-                                                                                   const GodConst32 &k32) {
-  return god32s<false>(m0, m1, m2, k32);
-}
-#define PDFS_LU64(MODE_, ARITH_, FN)                                                                  \
-  template <>                                                                                         \
-  __device__ __forceinline__ double local_update<double, MODE_, ARITH_, false>(                      \
-      double m0, double m1, double m2, const GodConst64 &k64, const GodConst32 &) {                  \
-    return FN(m0, m1, m2, k64);                                                                       \
-  }
-PDFS_LU64(MODE_MIN, ARITH_REF, god_ref64)
-PDFS_LU64(MODE_MIN, ARITH_FAST, god_fast64)
-PDFS_LU64(MODE_REPLACE, ARITH_REF, god_ref64)
-PDFS_LU64(MODE_REPLACE, ARITH_FAST, god_fast64)
-#undef PDFS_LU64
-#define PDFS_LUMX(MODE_, ISO_)                                                                       \
-  template <>                                                                                       \
-  __device__ __forceinline__ double local_update<double, MODE_, ARITH_MIXED, ISO_>(                 \
-      double m0, double m1, double m2, const GodConst64 &, const GodConst32 &k32) {                 \
-    return god_mixed64<ISO_>(m0, m1, m2, k32);                                                      \
-  }
-PDFS_LUMX(MODE_MIN, true)
-PDFS_LUMX(MODE_MIN, false)
-PDFS_LUMX(MODE_REPLACE, true)
-PDFS_LUMX(MODE_REPLACE, false)
-#undef PDFS_LUMX
-#define PDFS_LUPR(MODE_, ISO_)                                                                       \
-  template <>                                                                                       \
-  __device__ __forceinline__ double local_update<double, MODE_, ARITH_PAIR, ISO_>(                  \
-      double m0, double m1, double m2, const GodConst64 &, const GodConst32 &k32) {                 \
-    return god_pair<ISO_>(m0, m1, m2, k32);                                                         \
-  }
-PDFS_LUPR(MODE_MIN, true)
-PDFS_LUPR(MODE_MIN, false)
-PDFS_LUPR(MODE_REPLACE, true)
-PDFS_LUPR(MODE_REPLACE, false)
-#undef PDFS_LUPR
 
 // Records a timeout and raises the abort flags (global and CTA).
 __device__ __forceinline__ void raise_timeout(const SweepArgs &a, int col, volatile int *s_abort) {
@@ -438,6 +421,64 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned parity, const Sw
       return false;
     }
   }
+}
+
+// ---- faces handed over by mail (pencils and bricks) ----
+__device__ __forceinline__ void st_relaxed_gpu_u64(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+// A value's 32-bit pieces, each tagged with the epoch in the upper word.
+template <class T>
+__device__ __forceinline__ void mail_put(unsigned long long *e, T v, int epoch) {
+  const unsigned long long tag = (unsigned long long)(unsigned)epoch << 32;
+  if constexpr (sizeof(T) == 4) {
+    st_relaxed_gpu_u64(e, tag | __float_as_uint(v));
+  } else {
+    st_relaxed_gpu_u64(e, tag | (unsigned)__double2loint(v));
+    st_relaxed_gpu_u64(e + 1, tag | (unsigned)__double2hiint(v));
+  }
+}
+template <class T>
+__device__ __forceinline__ bool mail_get(const unsigned long long *e, int epoch, T &v) {
+  const unsigned tag = (unsigned)epoch;
+  const unsigned long long w0 = ld_relaxed_gpu_u64(e);
+  if constexpr (sizeof(T) == 4) {
+    v = __uint_as_float((unsigned)w0);
+    return (unsigned)(w0 >> 32) == tag;
+  } else {
+    const unsigned long long w1 = ld_relaxed_gpu_u64(e + 1);
+    v = __hiloint2double((int)(unsigned)w1, (int)(unsigned)w0);
+    return (unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 32) == tag;
+  }
+}
+// One idle round of a helper warp: lane 0 decides, for the whole warp, to give
+// up on the abort flag or after wait_cycles without progress.
+__device__ __forceinline__ bool helper_idle(const SweepArgs &a, int col, volatile int *s_abort, long long t_last,
+                                            unsigned &nap) {
+  int stop = 0;
+  if ((threadIdx.x & 31) == 0) {
+    if (*s_abort || *(volatile int *)(a.err + 1)) {
+      stop = 1;
+    } else if (cycles() - t_last > a.wait_cycles) {
+      raise_timeout(a, col, s_abort);
+      stop = 1;
+    }
+  }
+  if (__shfl_sync(0xffffffffu, stop, 0)) {
+    *s_abort = 1;
+    return true;
+  }
+  if (nap) __nanosleep(nap);
+  nap = min(nap + 32u, 128u);
+  return false;
+}
+__device__ __forceinline__ void fence_proxy_async_global() {
+  asm volatile("fence.proxy.async.global;\n" ::: "memory");
 }
 
 template <class T, int TY, int R, int MODE, int ARITH, bool ISO>

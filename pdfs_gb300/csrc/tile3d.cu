@@ -27,8 +27,8 @@ std::vector<int> brick_order(int ntx, int nty, int ntz) {
 
 template <class T, int BY, int BZ, int MODE, int ARITH, bool ISO>
 static cudaError_t launch_t3(const SweepArgs &a, const Layout &L, int sms, cudaStream_t st, int *grid_used) {
-  using G = T3Geo<T, BY, BZ>;
-  auto kern = t3_sweep_kernel<T, BY, BZ, MODE, ARITH, ISO>;
+  using G = T3Geo<T, 16, BY, BZ>;
+  auto kern = t3_sweep_kernel<T, 16, BY, BZ, MODE, ARITH, ISO>;
   CUtensorMap m;
   cudaError_t e = encode_field_map(&m, a.u, sizeof(T), L, a.nz + 2, G::W, G::RY, G::RZ);
   if (e != cudaSuccess) return e;
@@ -269,8 +269,8 @@ int octant_scratch_ints(int ntx, int nty, int ntz) {
 
 template <class T, int BZ, int MODE, int ARITH, bool ISO>
 static cudaError_t launch_oct(const SweepArgs &a, const Layout &L, int sms, cudaStream_t st, int *grid_used) {
-  using G = T3Geo<T, 16, BZ>;
-  auto kern = t3_sweep_kernel<T, 16, BZ, MODE, ARITH, ISO, true>;
+  using G = T3Geo<T, 16, 16, BZ>;
+  auto kern = t3_sweep_kernel<T, 16, 16, BZ, MODE, ARITH, ISO, true>;
   CUtensorMap m;
   cudaError_t e = encode_field_map(&m, a.u, sizeof(T), L, a.nz + 2, G::W, G::RY, G::RZ);
   if (e != cudaSuccess) return e;
@@ -295,7 +295,7 @@ cudaError_t launch_octant_round(int which, int arith, bool iso, int nsw, const S
   // rounds on 16^3 bricks, 8 CTAs per SM instead of 4, were measured slower
   // on the 768^3 grid: full round 22.4 -> 25.9 ms, masked 13.8 -> 15.0 ms.)
   const int bz = which == 0 ? 32 : 16;
-  if (!a0.tflag || !a0.torder || !a0.oct_bits || !a0.oct_tbits || a0.ntx < 1 || L.ty != 16 || L.tx != 16 ||
+  if (!a0.tflag || !a0.pmail || !a0.torder || !a0.oct_bits || !a0.oct_tbits || a0.ntx < 1 || L.ty != 16 || L.tx != 16 ||
       L.xo != 0 || which == 1 || (which == 2 && (!a0.bcap64 || !a0.bcap32)) || a0.ntz != (a0.nz + bz - 1) / bz ||
       nsw < 1 || nsw > kOctMax || (long long)a0.ntx * a0.nty * a0.ntz >= (1ll << 27))
     return cudaErrorInvalidValue;
@@ -354,7 +354,7 @@ cudaError_t launch_octant_round(int which, int arith, bool iso, int nsw, const S
 
 cudaError_t launch_sweep_bricks(int which, int by, int bz, int arith, bool iso, const SweepArgs &a0, const Layout &L,
                                 int sms, cudaStream_t st, int *g) {
-  if (!a0.tflag || !a0.torder || a0.ntx < 1 || a0.nty < 1 || a0.ntz < 1 || L.ty != by || L.tx != 16 ||
+  if (!a0.pmail || !a0.torder || a0.ntx < 1 || a0.nty < 1 || a0.ntz < 1 || L.ty != by || L.tx != 16 ||
       L.xo != 0 || (which == 2 && (!a0.bcap64 || !a0.bcap32)))
     return cudaErrorInvalidValue;
   SweepArgs a = a0;

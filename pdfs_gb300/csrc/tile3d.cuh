@@ -1,4 +1,4 @@
-// tile3d.cuh -- the 3-D tile sweep: each CTA sweeps a 16 x BY x BZ brick of
+// tile3d.cuh -- the 3-D tile sweep: each CTA sweeps a BX x BY x BZ brick of
 // the grid held whole in shared memory, hyperplane by hyperplane.
 //
 // The reference sweeps one hyperplane x+y+z = level of the whole grid per
@@ -10,25 +10,44 @@
 // twice over:
 //   * inside a brick, level by level: thread (lx, ly) -- brick-local
 //     coordinates in sweep order -- updates node (lx, ly, L - lx - ly) at
-//     level L, and a CTA barrier separates levels.  A level reads the
-//     previous level's results and the next level's old values straight from
-//     the shared-memory copy of the brick;
-//   * across bricks, by per-brick completion flags in global memory: a brick
-//     starts its levels once its (at most three) upwind bricks have published
-//     this sweep's epoch, and publishes its own after its stores are visible.
-//     Persistent CTAs take bricks by ticket in wavefront order (every upwind
-//     brick holds a smaller ticket), so the wait always ends.
+//     level L, from the previous level's results and the next level's old
+//     values in the shared-memory copy of the brick; one barrier a level.
+//     Columns are listed by diagonal lx + ly, so that a warp has a node to update
+//     on BZ + 2 to BZ + 7 levels;
+//   * across bricks, face by face: the threads on a brick's three downwind
+//     faces write their nodes' final values to a mailbox in global memory, each
+//     tagged with the sweep's epoch in one 64-bit word (a 64-bit store is
+//     single-copy atomic, so a reader that sees the tag sees the value: no
+//     fence, no counter).  A helper warp of the downwind brick polls those words,
+//     patches the values into the upwind halo of the brick's box and arrives on
+//     an mbarrier for every GL levels whose faces are there, so a brick runs some
+//     16 levels and an L2 round trip behind its upwind neighbours instead of a
+//     whole brick.  Persistent CTAs take bricks by ticket in wavefront order
+//     (every upwind brick holds a smaller ticket), so the wait always ends.
+//
+// What bounds it: the dependency chain.  Waiting for whole upwind bricks makes
+// a sweep (n/BX + n/BY + n/BZ) bricks of BX + BY + BZ - 2 levels deep, about 9n
+// levels; handing faces over level by level brings that to the sweep's own 3n
+// plus an L2 round trip per brick crossed.
+// Measured (octant rounds; FP32 full round / FP32 masked round / pair round): with
+// bricks that waited for whole upwind bricks, 768^3 22.0 / 13.0 / 20.5 ms, 320 x
+// 300 x 280 5.3 / 3.2 / 5.5 ms; handed over level by level, 23.6 / 9.5 / 16.7 and
+// 3.15 / 1.1 / 2.2 ms.  The 768^3 full round, which has bricks enough to fill the
+// chip, pays for the mail (issue slots are 56 % busy there); every grid with
+// fewer, and every masked round, gains.  Tried on the way: the helper stepping
+// through the levels' barrier (29.8 ms for the 768^3 full round), a second
+// helper warp sending the faces (27.9: 48 registers a thread, and the sender's
+// path was the level's), warps chained by mbarriers instead of a barrier a
+// level (34.4).
 //
 // A brick's old values do not depend on its upwind bricks, so its whole box
 // (the brick and a one-node halo, rows rounded up to 16 bytes) is requested
-// by one TMA copy as soon as the ticket is taken; only the upwind halo faces
-// are read again, from L2, after the flags.  Updated nodes are stored to
-// global memory as they are computed (unchanged nodes are not written).
-//
-// Against the column kernel (sweep.cuh) this trades the cross-column
-// mailboxes, the plane ring and the per-step warp hand-offs for one barrier
-// per level and a 1.5-2x halo read, and it keeps a brick's every level in
-// one CTA's shared memory.
+// by one TMA copy as soon as the ticket is taken.  A neighbour cannot
+// overwrite a value this brick still needs: a node next to one of this brick's
+// updated nodes waits for that node's mail, which is written after this
+// brick's box has landed.  New values stay in the box; the rows with a changed
+// node go to global memory at the brick's end, a row at a time (a store per
+// node as it is computed touches up to 32 lines a warp).
 //
 // Every wait is bounded (SweepArgs::wait_cycles): on expiry the kernel
 // records DEV_ERR_TIMEOUT, raises the abort flag, lets its own TMA copy land
@@ -38,30 +57,89 @@
 
 namespace pdfs {
 
-template <class T, int BY_, int BZ>
+template <class T, int BX_, int BY_, int BZ>
 struct T3Geo {
-  static constexpr int BX = 16, BY = BY_;
+  static constexpr int BX = BX_, BY = BY_;
   // box row: x0-1 .. x0+BX, rounded up to 16 bytes; the field's index has no
-  // x offset, so x0 - 1 = 16*bi starts the row on a 16-byte boundary
+  // x offset, so x0 - 1 = BX*bi starts the row on a 16-byte boundary
   static constexpr int W = (int)((((BX + 2) * sizeof(T)) + 15) / 16 * 16 / sizeof(T));
   static constexpr int RY = BY + 2;       // box rows: y0-1 .. y0+BY
   static constexpr int RZ = BZ + 2;       // box planes: z0-1 .. z0+BZ
   static constexpr int PL = RY * W;       // plane stride in shared memory
   static constexpr int NL = BX + BY + BZ - 2;  // levels of one brick
-  static constexpr int NT = BX * BY;      // one thread per (x, y) of the brick
-  static constexpr int NZB = BZ / 8;      // 8^3 scheduler blocks per brick column
+  static constexpr int NC = BX * BY;      // compute threads: one per (x, y) of the brick
+  static constexpr int NT = NC + 32;      // and a helper warp
+  static constexpr int WV = (int)sizeof(T) / 4;  // mailbox words per value (32 value bits each)
+  // mailbox of a brick: x face [(lz + ly) % BZ][ly], y face [(lz + lx) % BZ][lx],
+  // z face [(lx + ly) % BY][lx] -- one row per level of the reading brick, and
+  // (the modulus) no unused entries
+  static constexpr int MX = 0, MY = BZ * BY, MZ = MY + BZ * BX, MAIL = MZ + BX * BY;
+  static constexpr int SL = sizeof(T) == 4 ? 4 : 2;  // levels polled at a time
+  static constexpr int NBX = BX / 8, NBY = BY / 8, NZB = BZ / 8;  // 8^3 scheduler blocks per brick
+  static constexpr int NB = NBX * NBY * NZB;
   static constexpr unsigned BOX_BYTES = (unsigned)(W * RY * RZ * sizeof(T));
   static constexpr size_t OFF_MASK = ((size_t)BOX_BYTES + 127) & ~size_t(127);
-  static constexpr size_t OFF_BAR = OFF_MASK + (size_t)BZ * BY * 4;
-  static constexpr size_t BYTES = OFF_BAR + 16;
-  static_assert(BZ % 8 == 0 && BY % 8 == 0, "bricks hold whole 8^3 blocks");
-  static constexpr int NBX = BX / 8, NBY = BY / 8;  // 8^3 blocks per brick in x and y
+  using PlaneBits = typename std::conditional<(BZ > 32), unsigned long long, unsigned>::type;  // one bit per plane
+  static constexpr size_t OFF_CHG = OFF_MASK + (size_t)BZ * BY * 4;
+  static constexpr size_t OFF_BAR = OFF_CHG + (size_t)NC * sizeof(PlaneBits);
+  // the box's barrier, then one per GL levels (their upwind faces are there)
+  static constexpr int GL = 4, NG = (NL + GL - 1) / GL;
+  static constexpr size_t BYTES = OFF_BAR + 8 + (size_t)NG * 8;
+  // resident CTAs asked of the compiler: what shared memory allows, at most 4
+  // (56 registers a thread: 3 CTAs with more cost the 768^3 rounds 4 to 9 %)
+  static constexpr int CTAS = 227 * 1024 / (int)(BYTES + 1536) < 4 ? 227 * 1024 / (int)(BYTES + 1536) : 4;
+  using LevelBits = typename std::conditional<(NL > 64), unsigned __int128, unsigned long long>::type;  // one bit per level
+  __device__ static __forceinline__ int top(LevelBits b) {  // one past the highest bit
+    const unsigned long long lo = (unsigned long long)b;
+    if constexpr (sizeof(LevelBits) == 16) {
+      const unsigned long long hi = (unsigned long long)(b >> 64);
+      if (hi) return 128 - __clzll((long long)hi);
+    }
+    return lo ? 64 - __clzll((long long)lo) : 0;
+  }
+  // a column's planes as bits: sweep order <-> grid order
+  __device__ static __forceinline__ PlaneBits flip(PlaneBits b) {
+    if constexpr (BZ > 32)
+      return __brevll(b) >> (64 - BZ);
+    else
+      return __brev(b) >> (32 - BZ);
+  }
+  // bits [s, s + 32) of the planes (s may be negative), and back
+  __device__ static __forceinline__ unsigned level_word(PlaneBits b, int s) {
+    const unsigned long long w = b;
+    return s >= 64 || s <= -64 ? 0u : (unsigned)(s >= 0 ? w >> s : w << -s);
+  }
+  __device__ static __forceinline__ PlaneBits plane_bits(unsigned w, int s) {
+    const unsigned long long v = w;
+    return s >= 64 || s <= -64 ? PlaneBits(0) : PlaneBits(s >= 0 ? v << s : v >> -s);
+  }
+  static_assert(BZ % 8 == 0 && BY % 8 == 0 && BX % 8 == 0, "bricks hold whole 8^3 blocks");
+  static_assert(BX <= BZ && BY <= BZ, "x and y mailbox rows wrap at most once");
+  static_assert(BX + BY <= 32 && NB <= 32 && NZB * (NBX + NBY) + NBX * NBY <= 32, "one lane each");
   static_assert((W * sizeof(T)) % 16 == 0, "TMA rows are 16-byte multiples");
 };
 
-__device__ __forceinline__ void st_release_gpu(int *p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
+// The levels' barrier: the compute threads.
+template <int N>
+__device__ __forceinline__ void level_bar() {
+  asm volatile("bar.sync 1, %0;\n" ::"n"(N) : "memory");
 }
+
+// One ticket, decoded (shared memory; two slots, the next ticket's is filled
+// while a brick runs).
+struct T3Desc {
+  int stop;          // no ticket left, or the kernel is giving up
+  int li, lj, lk;    // the brick in sweep order
+  int sx, sy, sz;    // the sweep's directions
+  int sweep;         // OCT: which sweep of the round
+  int tile, epoch;   // the brick in grid order; the sweep's flag value and mail tag
+  unsigned long long *mail;  // the brick's mailbox
+  int lev0, lev1;    // its levels [lev0, lev1): those that reach its visited planes
+  // visited 8^3 blocks, one bit each: the brick's own (z, y, x; x fastest), and
+  // the ones across its upwind faces (x: z, y; y: z, x; z: y, x)
+  unsigned act, upx, upy, upz;
+};
+
 // A brick's completion: the CTA barrier before it orders every thread's
 // stores before thread 0's acquire-release fence at GPU scope, which orders
 // them before the relaxed flag store (the fence-then-relaxed-store pattern of
@@ -71,46 +149,300 @@ __device__ __forceinline__ void publish_gpu(int *p, int v) {
   asm volatile("st.relaxed.gpu.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
 
-// Column of thread tid when the brick's 16 x BY columns are listed by
-// diagonal d = lx + ly (then by ly).  Column (lx, ly) holds a node of level L
+// The brick's BX x BY columns are listed by diagonal d = lx + ly (then by
+// ly).  Column (lx, ly) holds a node of level L
 // for L - lx - ly in [0, BZ), so a warp whose 32 columns span diagonals
 // d0 .. d1 runs the level body on BZ + d1 - d0 levels: BZ + 2 to BZ + 7 for
 // 16 x 16 columns listed by diagonal, BZ + 16 for the row-major warp of two
 // rows (158 against 256 warp-level bodies per 16^3 brick).
 template <int BX, int BY>
-__device__ __forceinline__ int2 diag_column(int tid) {
-  int base = 0;
-#pragma unroll 1
-  for (int d = 0; d <= BX + BY - 2; ++d) {
-    const int lo = d - (BX - 1) > 0 ? d - (BX - 1) : 0, hi = d < BY - 1 ? d : BY - 1;  // ly on diagonal d
-    if (tid < base + hi - lo + 1) return make_int2(d - (lo + tid - base), lo + tid - base);
-    base += hi - lo + 1;
+__device__ __forceinline__ int diag_rank(int lx, int ly) {  // the position of column (lx, ly) in that order
+  constexpr int S = BX < BY ? BX : BY, M = BX < BY ? BY : BX;
+  const int d = lx + ly, t = BX + BY - 1 - d;
+  const int before = d <= S ? d * (d + 1) / 2 : d <= M ? S * (S + 1) / 2 + (d - S) * S : BX * BY - t * (t + 1) / 2;
+  return before + ly - max(0, d - (BX - 1));
+}
+
+// The ticket taken next, decoded into d by one warp.  Tickets of bricks
+// without a visited block are passed over (no brick waits for them).  In a
+// round, the brick and its six face neighbours have to finish their latest
+// earlier sweep first: lanes 0..6 leave in wait_flag a flag that is not there
+// yet (else -1), for t3_wait once the current brick has published its own.
+template <class G, bool OCT>
+__device__ __forceinline__ void t3_next(const SweepArgs &a, int ntile, T3Desc &d, volatile int *s_abort,
+                                        int &wait_flag, int &wait_epoch) {
+  const int lane = threadIdx.x & 31;
+  const int ntx = a.ntx, nty = a.nty, ntz = a.ntz;
+  wait_flag = -1;
+  for (;;) {
+    int tk = 0;
+    if (lane == 0) tk = (*s_abort || *(volatile int *)(a.err + 1)) ? ntile : atomicAdd(a.ticket, 1);
+    tk = __shfl_sync(0xffffffffu, tk, 0);
+    if (tk >= ntile) {
+      if (lane == 0) d.stop = 1;
+      break;
+    }
+    int lt = __ldg(a.torder + tk), osw = 0;  // OCT: (sweep << 27) | brick, else the brick, in sweep order
+    int sx = a.sx, sy = a.sy, sz = a.sz;
+    unsigned obit = 0;   // OCT: the ordering's bit
+    bool every = false;  // the sweep visits every block
+    if constexpr (OCT) {
+      osw = lt >> 27;
+      lt &= 0x07ffffff;
+      const int sn = (a.oct_first + osw) % 8 + 1;
+      obit = 1u << (sn - 1);
+      every = (a.oct_full >> osw) & 1u;
+      ordering_signs(sn, &sx, &sy, &sz);
+    } else {
+      every = a.blk_active == nullptr;
+    }
+    const int li = lt % ntx, lj = (lt / ntx) % nty, lk = lt / (ntx * nty);
+    const int bi = sx > 0 ? li : ntx - 1 - li, bj = sy > 0 ? lj : nty - 1 - lj, bk = sz > 0 ? lk : ntz - 1 - lk;
+    const int tile = (bk * nty + bj) * ntx + bi;
+    const int bx0 = G::NBX * bi, by0 = G::NBY * bj, bz0 = G::NZB * bk;  // the brick's first block
+    auto visited = [&](int bx, int by, int bz) -> bool {
+      if (bx < 0 || by < 0 || bz < 0 || bx >= a.nbx || by >= a.nby || bz >= a.nbz) return false;
+      const long long b = ((long long)bz * a.nby + by) * a.nbx + bx;
+      if constexpr (OCT)
+        return every || (__ldg(a.oct_bits + b) & obit) != 0;
+      else
+        return every || __ldg(a.blk_active + b) != 0;
+    };
+    bool on = false;
+    if (lane < G::NB)
+      on = visited(bx0 + lane % G::NBX, by0 + (lane / G::NBX) % G::NBY, bz0 + lane / (G::NBX * G::NBY));
+    const unsigned act = __ballot_sync(0xffffffffu, on);
+    if (act == 0) continue;
+    constexpr int UX = G::NBY * G::NZB, UY = G::NBX * G::NZB, UZ = G::NBX * G::NBY;
+    on = false;
+    if (lane < UX) {
+      on = li > 0 && visited(sx > 0 ? bx0 - 1 : bx0 + G::NBX, by0 + lane % G::NBY, bz0 + lane / G::NBY);
+    } else if (lane < UX + UY) {
+      const int i = lane - UX;
+      on = lj > 0 && visited(bx0 + i % G::NBX, sy > 0 ? by0 - 1 : by0 + G::NBY, bz0 + i / G::NBX);
+    } else if (lane < UX + UY + UZ) {
+      const int i = lane - UX - UY;
+      on = lk > 0 && visited(bx0 + i % G::NBX, by0 + i / G::NBX, sz > 0 ? bz0 - 1 : bz0 + G::NZB);
+    }
+    const unsigned up = __ballot_sync(0xffffffffu, on);
+    if constexpr (OCT) {
+      // the round's earlier sweeps, lanes 0..6: the brick, then its neighbours
+      if (lane < 7) {
+        int n = -1;
+        if (lane == 0) n = tile;
+        if (lane == 1 && bi > 0) n = tile - 1;
+        if (lane == 2 && bi < ntx - 1) n = tile + 1;
+        if (lane == 3 && bj > 0) n = tile - ntx;
+        if (lane == 4 && bj < nty - 1) n = tile + ntx;
+        if (lane == 5 && bk > 0) n = tile - ntx * nty;
+        if (lane == 6 && bk < ntz - 1) n = tile + ntx * nty;
+        int need = -1;
+        if (n >= 0) {
+          const unsigned tb = __ldg(a.oct_tbits + n);
+          for (int j = osw - 1; j >= 0 && need < 0; --j)
+            if (((a.oct_full >> j) & 1u) || ((tb >> ((a.oct_first + j) % 8)) & 1u)) need = j;
+        }
+        // (the CTA's current brick may be among them: looked at here, waited for later)
+        if (need >= 0 && ld_acquire_gpu(a.tflag + n) < a.epoch + need) {
+          wait_flag = n;
+          wait_epoch = a.epoch + need;
+        }
+      }
+      __syncwarp();
+    }
+    if (lane == 0) {
+      // the planes of the brick's visited blocks, in sweep order
+      unsigned zb = 0;
+#pragma unroll
+      for (int q = 0; q < G::NZB; ++q)
+        if ((act >> (q * UZ)) & ((1u << UZ) - 1u)) zb |= 1u << q;
+      const int q0 = __ffs(zb) - 1, q1 = 31 - __clz(zb);
+      const int lo = sz > 0 ? 8 * q0 : 8 * (G::NZB - 1 - q1), hi = sz > 0 ? 8 * q1 + 7 : 8 * (G::NZB - 1 - q0) + 7;
+      d.stop = 0;
+      d.li = li;
+      d.lj = lj;
+      d.lk = lk;
+      d.sx = sx;
+      d.sy = sy;
+      d.sz = sz;
+      d.sweep = osw;
+      d.tile = tile;
+      d.epoch = OCT ? a.epoch + osw : a.epoch;
+      d.mail = a.pmail + (size_t)tile * (G::MAIL * G::WV);
+      d.lev0 = lo;                                    // column (0, 0) reaches the first visited plane
+      d.lev1 = min(G::NL, hi + G::BX + G::BY - 1);    // the last column leaves the last one
+      d.act = act;
+      d.upx = up & ((1u << UX) - 1u);
+      d.upy = (up >> UX) & ((1u << UY) - 1u);
+      d.upz = (up >> (UX + UY)) & ((1u << UZ) - 1u);
+    }
+    break;
   }
-  return make_int2(0, 0);
+  __syncwarp();
+}
+
+// Waits (bounded) for the flag that t3_next left.
+__device__ __forceinline__ void t3_wait(const SweepArgs &a, int wait_flag, int wait_epoch, volatile int *s_abort) {
+  if (wait_flag >= 0 && ld_acquire_gpu(a.tflag + wait_flag) < wait_epoch) {
+    const long long t0 = cycles();
+    unsigned nap = 32;
+    while (ld_acquire_gpu(a.tflag + wait_flag) < wait_epoch) {
+      if (*s_abort || *(volatile int *)(a.err + 1)) {
+        *s_abort = 1;
+        break;
+      }
+      if (cycles() - t0 > a.wait_cycles) {
+        raise_timeout(a, wait_flag, s_abort);
+        break;
+      }
+      __nanosleep(nap);
+      nap = min(nap * 2, 256u);
+    }
+  }
+  __syncwarp();
+}
+
+// A mailbox entry as loaded: a tagged word per 32 value bits.
+template <class T>
+struct Mail {
+  unsigned long long w[sizeof(T) / 4];
+  __device__ __forceinline__ void load(const unsigned long long *e) {
+    if constexpr (sizeof(T) == 4)
+      w[0] = ld_relaxed_gpu_u64(e);
+    else
+      asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];\n" : "=l"(w[0]), "=l"(w[1]) : "l"(e) : "memory");
+  }
+  __device__ __forceinline__ bool tagged(int epoch) const {
+    bool ok = (unsigned)(w[0] >> 32) == (unsigned)epoch;
+    if constexpr (sizeof(T) == 8) ok = ok && (unsigned)(w[1] >> 32) == (unsigned)epoch;
+    return ok;
+  }
+  __device__ __forceinline__ T value() const {
+    if constexpr (sizeof(T) == 4)
+      return __uint_as_float((unsigned)w[0]);
+    else
+      return __hiloint2double((int)(unsigned)w[1], (int)(unsigned)w[0]);
+  }
+};
+
+// The helper's receiving: lanes [0, BY) the x-face rows and [BY, BY + BX)
+// the y-face columns, and (a second set) lanes [0, BX) the z-face columns.  A
+// lane reads position p of its row or column k at level k + p: p runs along z
+// for the x and y faces, along y for the z face.  It polls SL levels at a time,
+// as far ahead of the compute warps as the mail is there, patches the values
+// into the box and arrives on the barrier of each group of GL levels.  Mail is
+// awaited where the upwind brick's 8^3 block and mine are both visited: other
+// halo values are the box's own.
+template <class T, class G>
+__device__ __forceinline__ void t3_receive(const SweepArgs &a, const T3Desc &d, int tile, int epoch, T *box, int x0,
+                                           int y0, int zcnt, uint64_t *grp, volatile int *s_abort) {
+  constexpr int BX = G::BX, BY = G::BY, BZ = G::NZB * 8, W = G::W, PL = G::PL;
+  using LevelBits = typename G::LevelBits;
+  const int lane = threadIdx.x & 31;
+  const bool px = d.sx > 0, py = d.sy > 0, pz = d.sz > 0;
+  const bool xf = lane < BY, yf = !xf && lane < BY + BX;
+  const int k = xf ? lane : lane - BY;
+  const int ku = xf ? (py ? k : BY - 1 - k) : (px ? k : BX - 1 - k), zu = px ? lane : BX - 1 - lane;  // in grid order
+  // awaited levels, one bit each
+  LevelBits nf = 0, nz = 0;
+  if (xf ? d.li > 0 && y0 + ku <= a.ny : yf && d.lj > 0 && x0 + ku <= a.nx) {
+#pragma unroll
+    for (int q = 0; q < G::NZB; ++q) {
+      const int c8 = min(8, zcnt - 8 * q);
+      if (c8 <= 0) break;
+      const unsigned mine = xf ? d.act >> ((q * G::NBY + (ku >> 3)) * G::NBX + (px ? 0 : G::NBX - 1))
+                               : d.act >> ((q * G::NBY + (py ? 0 : G::NBY - 1)) * G::NBX + (ku >> 3));
+      const unsigned theirs = xf ? d.upx >> (q * G::NBY + (ku >> 3)) : d.upy >> (q * G::NBX + (ku >> 3));
+      if (mine & theirs & 1u) nf |= LevelBits((1u << c8) - 1u) << (k + (pz ? 8 * q : BZ - 8 * q - c8));
+    }
+  }
+  if (lane < BX && d.lk > 0 && x0 + zu <= a.nx) {
+#pragma unroll
+    for (int q = 0; q < G::NBY; ++q) {
+      const int c8 = min(8, a.ny - y0 + 1 - 8 * q);
+      if (c8 <= 0) break;
+      const unsigned mine = d.act >> (((pz ? 0 : G::NZB - 1) * G::NBY + q) * G::NBX + (zu >> 3));
+      if (mine & (d.upz >> (q * G::NBX + (zu >> 3))) & 1u)
+        nz |= LevelBits((1u << c8) - 1u) << (lane + (py ? 8 * q : BY - 8 * q - c8));
+    }
+  }
+  const int lev0 = d.lev0, lev1 = d.lev1;
+  // past the last awaited level every level is ready
+  const int gend = min(lev1, __reduce_max_sync(0xffffffffu, max(G::top(nf), G::top(nz))));
+  // mail of level lv: row lv (mod the face's rows) of the upwind brick's face
+  const long long upf = xf ? tile - d.sx : tile - d.sy * a.ntx, upz = tile - d.sz * a.ntx * a.nty;
+  const unsigned long long *mf = a.pmail + (upf * G::MAIL + (xf ? G::MX : G::MY) + k) * G::WV;
+  const unsigned long long *mz = a.pmail + (upz * G::MAIL + G::MZ + lane) * G::WV;
+  const int fcols = (xf ? BY : BX) * G::WV;
+  // box element read at level 0 and the step per level
+  const int fs = pz ? PL : -PL, zs = py ? W : -W;
+  T *bf = box + (pz ? 1 : BZ) * PL + (xf ? (1 + ku) * W + (px ? 0 : BX + 1) : (py ? 0 : BY + 1) * W + 1 + ku) - k * fs;
+  T *bz = box + (pz ? 0 : BZ + 1) * PL + (py ? 1 : BY) * W + 1 + zu - lane * zs;
+  constexpr int SL = G::SL;
+  bool live = true;  // false: gave up; the compute threads run out their levels (the call returns an error)
+  for (int g = 0; g < G::NG; ++g) {
+    const int g0 = max(lev0, g * G::GL), g1 = min(gend, g * G::GL + G::GL);
+    for (int L = g0; L < g1 && live; L += SL) {
+      Mail<T> v[SL], w[SL];
+      const long long t_last = cycles();
+      unsigned nap = 0;
+      for (;;) {
+        bool ok = true;
+#pragma unroll
+        for (int i = 0; i < SL; ++i) {  // all the loads first: they are in flight together
+          const int lv = L + i;
+          if (lv < g1 && ((nf >> lv) & 1u)) v[i].load(mf + (lv >= BZ ? lv - BZ : lv) * fcols);
+          if (lv < g1 && ((nz >> lv) & 1u)) w[i].load(mz + (lv % BY) * (BX * G::WV));
+        }
+#pragma unroll
+        for (int i = 0; i < SL; ++i) {
+          const int lv = L + i;
+          if (lv < g1 && ((nf >> lv) & 1u)) ok = ok && v[i].tagged(epoch);
+          if (lv < g1 && ((nz >> lv) & 1u)) ok = ok && w[i].tagged(epoch);
+        }
+        if (__all_sync(0xffffffffu, ok)) break;
+        if (helper_idle(a, tile, s_abort, t_last, nap)) {
+          live = false;
+          break;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < SL; ++i) {
+        const int lv = L + i;
+        if (lv < g1 && ((nf >> lv) & 1u)) bf[lv * fs] = v[i].value();
+        if (lv < g1 && ((nz >> lv) & 1u)) bz[lv * zs] = w[i].value();
+      }
+      __syncwarp();
+    }
+    if (lane == 0) mbar_arrive(grp + g);
+  }
 }
 
 // OCT: an octant round -- up to kOctMax sweeps in one launch (a cycle of the
-// 8 orderings).  A ticket
-// names (sweep j, brick); ordering (oct_first + j) % 8 + 1 visits the bricks
-// and blocks whose bits name it, or every brick when bit j of oct_full is
-// set.  Before its box is read, a
-// brick waits until it and its six face neighbours have finished their latest
-// earlier sweep of the round (their values are this sweep's old values), then
-// for its upwind bricks in this sweep as usual.  Flags carry epoch + j, so
+// 8 orderings).  A ticket names (sweep j, brick); ordering (oct_first + j) % 8 + 1
+// visits the bricks and blocks whose bits name it, or every brick when bit j
+// of oct_full is set.  Before its box is read, a brick waits until it and its six face neighbours have finished their latest
+// earlier sweep of the round (their values are this sweep's old values); its
+// upwind faces of this sweep come by mail as usual.  Flags carry epoch + j, so
 // "finished sweep j" is a flag >= epoch + j; the ticket list (k_oct_plan,
 // k_oct_merge) interleaves the sweeps by wavefront level with every brick
 // after the ones it waits on, so every wait is on a smaller ticket.  The
 // result is the sequential sweeps', bit for bit.
-template <class T, int BY_, int BZ, int MODE, int ARITH, bool ISO, bool OCT = false>
-__global__ void __launch_bounds__(16 * BY_) t3_sweep_kernel(const __grid_constant__ CUtensorMap tm_u,
-                                                            const __grid_constant__ SweepArgs a) {
-  using G = T3Geo<T, BY_, BZ>;
-  constexpr int BX = G::BX, BY = G::BY, W = G::W, PL = G::PL, NL = G::NL, NZB = G::NZB;
+template <class T, int BX_, int BY_, int BZ, int MODE, int ARITH, bool ISO, bool OCT = false>
+__global__ void __launch_bounds__(T3Geo<T, BX_, BY_, BZ>::NT,
+                                  (sizeof(T) == 4 || ARITH == ARITH_PAIR) ? T3Geo<T, BX_, BY_, BZ>::CTAS : 2)
+    t3_sweep_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ SweepArgs a) {
+  using G = T3Geo<T, BX_, BY_, BZ>;
+  using PlaneBits = typename G::PlaneBits;
+  constexpr int BX = G::BX, BY = G::BY, W = G::W, PL = G::PL, NZB = G::NZB;
   extern __shared__ __align__(1024) unsigned char sm[];
   T *box = reinterpret_cast<T *>(sm);
   uint32_t *smask = reinterpret_cast<uint32_t *>(sm + G::OFF_MASK);  // [BZ][BY] frozen words of the brick
-  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + G::OFF_BAR);
-  __shared__ int s_next, s_lo, s_hi;  // s_lo / s_hi: a masked brick's active planes (sweep order)
+  PlaneBits *schgp = reinterpret_cast<PlaneBits *>(sm + G::OFF_CHG);  // [BY][BX] planes changed (grid order)
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + G::OFF_BAR), *grp = bar + 1;
+  __shared__ T3Desc s_desc[2];
+  __shared__ unsigned long long s_max[OCT ? 8 : 1];  // per sweep: the CTA's change word
+  __shared__ unsigned s_chg[OCT ? 1 : G::NB];        // block-change output: the brick's blocks
   __shared__ volatile int s_abort;
 
   if ((saddr(sm) & 127u) != 0) {  // TMA destinations must be 128-byte aligned
@@ -121,379 +453,288 @@ __global__ void __launch_bounds__(16 * BY_) t3_sweep_kernel(const __grid_constan
     return;
   }
   const int tid = threadIdx.x, lane = tid & 31;
-  // brick-local x, y in sweep order; an octant round orders them by diagonal
-  const int lx = OCT ? diag_column<BX, BY>(tid).x : tid & (BX - 1);
-  const int ly = OCT ? diag_column<BX, BY>(tid).y : tid / BX;
-  int sxd = a.sx, syd = a.sy, szd = a.sz;  // OCT: set per ticket
-  int gxl = sxd > 0 ? lx : BX - 1 - lx;      // brick-local x, y in grid order
-  int gyl = syd > 0 ? ly : BY - 1 - ly;
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const int ntx = a.ntx, nty = a.nty, ntz = a.ntz;
+  const bool compute = tid < G::NC;
   // a block-masked sweep takes tickets only for the bricks with an active block
-  const int ntile = a.nticket ? *a.nticket : ntx * nty * ntz;
-  const uint8_t *__restrict__ tact = a.tact;
-  const long long plane = a.plane, px = a.px;
-  const float hmin = a.hmin;
-  const GodConst64 k64 = a.k64;
-  const GodConst32 k32 = a.k32;
-  const uint8_t *__restrict__ blk_active = a.blk_active;
-  unsigned int *__restrict__ blk_chg = a.blk_chg;
+  const int ntile = a.nticket ? *a.nticket : a.ntx * a.nty * a.ntz;
   const bool masked = a.fmask != nullptr;
   T *__restrict__ u = reinterpret_cast<T *>(a.u);
   const T *__restrict__ capg = reinterpret_cast<const T *>(a.cap);
-  int epoch = a.epoch;  // OCT: epoch + the ticket's sweep
-  T tmax = T(0);
 
   if (tid == 0) {
     s_abort = 0;
     mbar_init(bar, 1);
+    for (int g = 0; g < G::NG; ++g) mbar_init(grp + g, 1);
     mbar_fence_init();
-    s_next = atomicAdd(a.ticket, 1);
   }
+  __shared__ uint8_t s_col[G::NC];  // diagonal order -> ly * BX + lx
+  if (compute) s_col[diag_rank<BX, BY>(tid % BX, tid / BX)] = (uint8_t)tid;
+  if (tid < (OCT ? 8 : 1)) s_max[tid] = 0;
+  if (!OCT && tid < G::NB) s_chg[tid] = 0;
   __syncthreads();
-  unsigned par = 0;  // phase parity of the box barrier
-  for (;;) {
-    const int tk = s_next;
-    if (tid == 0) {
-      s_lo = BZ;
-      s_hi = -1;
-    }
-    // a uniform decision (s_abort may change under the reads); the barrier
-    // also orders every read of s_next before its next write
-    if (__syncthreads_or(tk >= ntile || s_abort)) break;
-    int lt, osw = 0;
-    unsigned obit = 0;   // OCT: the ticket's ordering bit
-    bool sfull = false;  // OCT: the ticket's sweep visits every block
-    if constexpr (OCT) {  // (sweep << 27) | brick in sweep order
-      const int e = a.torder[tk];
-      osw = e >> 27;
-      lt = e & 0x07ffffff;
-      sfull = (a.oct_full >> osw) & 1u;
-      const int sn = (a.oct_first + osw) % 8 + 1;
-      obit = 1u << (sn - 1);
-      ordering_signs(sn, &sxd, &syd, &szd);
-      gxl = sxd > 0 ? lx : BX - 1 - lx;
-      gyl = syd > 0 ? ly : BY - 1 - ly;
-      epoch = a.epoch + osw;
-    } else {
-      lt = a.torder[tk];  // local brick id in sweep order: (lk * nty + lj) * ntx + li
-    }
-    const int li = lt % ntx, lj = (lt / ntx) % nty, lk = lt / (ntx * nty);
-    const int bi = sxd > 0 ? li : ntx - 1 - li;
-    const int bj = syd > 0 ? lj : nty - 1 - lj;
-    const int bk = szd > 0 ? lk : ntz - 1 - lk;
-    const int tile = (bk * nty + bj) * ntx + bi;
+  int wait_flag = -1, wait_epoch = 0;  // helper warp: an earlier sweep's flag to wait for
+  if (!compute) t3_next<G, OCT>(a, ntile, s_desc[0], &s_abort, wait_flag, wait_epoch);
+  __syncthreads();
+
+  // my column, brick-local x, y in sweep order, by diagonal
+  const int col = compute ? s_col[tid] : 0, lx = col % BX, ly = col / BX, lxy = lx + ly;
+  for (int it = 0;; ++it) {
+    const T3Desc &d = s_desc[it & 1];
+    if (d.stop) break;
+    const int sxd = d.sx, syd = d.sy, szd = d.sz;
+    const int bi = sxd > 0 ? d.li : a.ntx - 1 - d.li;
+    const int bj = syd > 0 ? d.lj : a.nty - 1 - d.lj;
+    const int bk = szd > 0 ? d.lk : a.ntz - 1 - d.lk;
+    const int tile = d.tile;
     const int x0 = 1 + bi * BX, y0 = 1 + bj * BY, z0 = 1 + bk * BZ;
-
-    // block mask: a brick none of whose 8^3 blocks is active keeps its values
-    // and publishes at once (its faces are the old values its neighbours need);
-    // otherwise only the levels that reach its active planes run
-    bool run = true;
-    int lev0 = 0, lev1 = NL;  // levels [lev0, lev1) of this brick
-    if (OCT || blk_active) {
-      bool act = false;
-      if (tid < G::NBX * G::NBY * NZB) {
-        const int q = tid / (G::NBX * G::NBY);
-        const int bx = G::NBX * bi + tid % G::NBX, by = G::NBY * bj + (tid / G::NBX) % G::NBY;
-        const int bz = bk * NZB + q;
-        if (bx < a.nbx && by < a.nby && bz < a.nbz)
-          act = OCT ? sfull || (__ldg(a.oct_bits + ((long long)bz * a.nby + by) * a.nbx + bx) & obit) != 0
-                    : __ldg(blk_active + ((long long)bz * a.nby + by) * a.nbx + bx) != 0;
-        if (act) {  // the block's planes 8q .. 8q+7 (grid order) in sweep order
-          const int lo = szd > 0 ? 8 * q : BZ - 8 * q - 8;
-          atomicMin(&s_lo, lo);
-          atomicMax(&s_hi, lo + 7);
-        }
-      }
-      run = __syncthreads_or(act) != 0;
-      lev0 = s_lo;                        // thread (0, 0) reaches the first active plane
-      lev1 = min(NL, s_hi + BX + BY - 1);  // thread (15, 15) leaves the last one
-    }
-    if (tid == 32) s_next = atomicAdd(a.ticket, 1);  // the next brick's ticket, fetched ahead
-    if (!run) {
-      if (tid == 0 && tile != a.poison_col) st_release_gpu(a.tflag + tile, epoch);
-      __syncthreads();
-      continue;
-    }
-
+    const int zcnt = min(BZ, a.nz - z0 + 1);  // planes of the brick inside the grid
+    // the box: TMA from (x0 - 1, y0 - 1, z0 - 1); out-of-range rows and planes
+    // read 0 (never used).  The barrier before orders this CTA's generic accesses
+    // to the box (each thread's proxy fence) before the copy's writes; the global
+    // fence orders the flags acquired by this warp before the copy's reads.
     if constexpr (OCT) {
-      // the round's earlier sweeps: this brick and its six face neighbours
-      // (lanes 0..6 of warp 0, one each) finish their latest earlier sweep first
-      bool okp = true;
-      if (tid < 7) {
-        int n = -1;
-        if (tid == 0) n = tile;
-        if (tid == 1 && bi > 0) n = tile - 1;
-        if (tid == 2 && bi < ntx - 1) n = tile + 1;
-        if (tid == 3 && bj > 0) n = tile - ntx;
-        if (tid == 4 && bj < nty - 1) n = tile + ntx;
-        if (tid == 5 && bk > 0) n = tile - ntx * nty;
-        if (tid == 6 && bk < ntz - 1) n = tile + ntx * nty;
-        int need = -1;
-        if (n >= 0) {
-          const unsigned tb = __ldg(a.oct_tbits + n);
-          for (int j = osw - 1; j >= 0 && need < 0; --j)
-            if (((a.oct_full >> j) & 1u) || ((tb >> ((a.oct_first + j) % 8)) & 1u)) need = j;
-        }
-        if (need >= 0 && ld_acquire_gpu(a.tflag + n) < a.epoch + need) {
-          const long long t0 = cycles();
-          unsigned nap = 32;
-          while (ld_acquire_gpu(a.tflag + n) < a.epoch + need) {
-            if (s_abort || *(volatile int *)(a.err + 1)) {
-              s_abort = 1;
-              okp = false;
-              break;
-            }
-            if (cycles() - t0 > a.wait_cycles) {
-              raise_timeout(a, tile, &s_abort);
-              okp = false;
-              break;
-            }
-            __nanosleep(nap);
-            nap = min(nap * 2, 256u);
-          }
-        }
-      }
-      if (!__syncthreads_and(okp)) break;
+      if (!compute) t3_wait(a, wait_flag, wait_epoch, &s_abort);
     }
-    // the box: TMA from (x0 - 1, y0 - 1, z0 - 1); out-of-range rows and planes read 0 (never used)
-    fence_proxy_async();  // this CTA's generic accesses to the box come before the copy's writes
-    __syncthreads();
-    if (tid == 0) {
+    if (tid == G::NC) {
+      if constexpr (OCT) fence_proxy_async_global();
       mbar_arrive_tx(bar, G::BOX_BYTES);
       tma_load_3d(box, &tm_u, bi * BX, y0 - 1, z0 - 1, bar);
     }
-    const bool vxy = (x0 + gxl <= nx) && (y0 + gyl <= ny);
-    const int zcnt = min(BZ, nz - z0 + 1);  // planes of the brick inside the grid
     // frozen words of the brick's rows: node bit (x0 - 1 + gx) & 31
+    const int mshift = (bi * BX) & 31;
+    bool frozen = false;  // does one of them freeze a node of the brick?
     if (masked) {
       for (int q = tid; q < BZ * BY; q += G::NT) {
         const int p = q / BY, r = q % BY;
         uint32_t w = 0;
-        if (p < zcnt && y0 + r <= ny)
-          w = __ldg(a.fmask + (long long)(z0 + p) * (a.mask_fy * a.mask_fw) + (long long)(bi >> 1) * a.mask_fy +
-                    (y0 - 1 + r));
+        if (p < zcnt && y0 + r <= a.ny)
+          w = __ldg(a.fmask + (long long)(z0 + p) * (a.mask_fy * a.mask_fw) +
+                    (long long)((bi * BX) >> 5) * a.mask_fy + (y0 - 1 + r));
         smask[q] = w;
+        frozen = frozen || ((w >> mshift) & ((1u << BX) - 1u)) != 0;
       }
     }
-    const int mshift = 16 * (bi & 1) + gxl;
-    // active 8^3 blocks of my (x, y) column, one bit per z block of the brick
-    unsigned actz = (1u << NZB) - 1u;
-    if ((OCT || blk_active) && vxy) {
-      actz = 0;
-      const int bx = (x0 - 1 + gxl) >> 3, by = (y0 - 1 + gyl) >> 3;
-#pragma unroll
-      for (int q = 0; q < NZB; ++q) {
-        const int bz = bk * NZB + q;
-        if (bz < a.nbz && (OCT ? sfull || (__ldg(a.oct_bits + ((long long)bz * a.nby + by) * a.nbx + bx) & obit) != 0
-                                : __ldg(blk_active + ((long long)bz * a.nby + by) * a.nbx + bx) != 0))
-          actz |= 1u << q;
-      }
-    }
-    const long long gbase = (long long)z0 * plane + (long long)(y0 + gyl) * px + (x0 + gxl);
+    const int gxl = sxd > 0 ? lx : BX - 1 - lx;  // my column in grid order
+    const int gyl = syd > 0 ? ly : BY - 1 - ly;
+    const bool vxy = compute && (x0 + gxl <= a.nx) && (y0 + gyl <= a.ny);
     // replace-update: the cap bounds of my column's 8^3 blocks in this brick
     using CB = CapBound<T, ARITH>;
-    typename CB::type bnd[NZB];
+    typename CB::type bnds[NZB];
 #pragma unroll
     for (int q = 0; q < NZB; ++q) {
-      bnd[q] = 0;
-      if (MODE == MODE_REPLACE && vxy && bk * NZB + q < a.nbz)
-        bnd[q] = CB::load(a, ((long long)(bk * NZB + q) * a.nby + ((y0 - 1 + gyl) >> 3)) * a.nbx + ((x0 - 1 + gxl) >> 3));
+      bnds[q] = 0;
+      if (MODE == MODE_REPLACE && vxy)
+        bnds[q] = bk * NZB + q >= a.nbz ? typename CB::type(INFINITY) : CB::load(a, ((long long)(bk * NZB + q) * a.nby + ((y0 - 1 + gyl) >> 3)) * a.nbx + ((x0 - 1 + gxl) >> 3));
     }
-
-    // wait for the upwind bricks (lanes 0..2 of warp 0, one each)
-    bool ok = true;
-    if (tid < 3) {
-      int up = -1;
-      if (tid == 0 && li > 0) up = tile - sxd;
-      if (tid == 1 && lj > 0) up = tile - syd * ntx;
-      if (tid == 2 && lk > 0) up = tile - szd * ntx * nty;
-      // an upwind brick without an active block keeps its values: nothing to wait for
-      if constexpr (OCT) {
-        if (up >= 0 && !sfull && !(__ldg(a.oct_tbits + up) & obit)) up = -1;
-      } else {
-        if (up >= 0 && tact && !tact[up]) up = -1;
+    // the box copy has landed (the helper's wait is bounded; on abort it lets it
+    // land all the same): the others wait for the helper at the barrier
+    if (!compute && !mbar_wait(bar, it & 1, a, tile, &s_abort)) {
+      const long long t0 = cycles();
+      while (!mbar_try(bar, it & 1) && cycles() - t0 < 4000000000ll) {
       }
-      if (up >= 0 && ld_acquire_gpu(a.tflag + up) < epoch) {
-        const long long t0 = cycles();
-        unsigned nap = 32;
-        while (ld_acquire_gpu(a.tflag + up) < epoch) {
-          if (s_abort || *(volatile int *)(a.err + 1)) {
-            s_abort = 1;
-            ok = false;
-            break;
-          }
-          if (cycles() - t0 > a.wait_cycles) {
-            raise_timeout(a, tile, &s_abort);
-            ok = false;
-            break;
-          }
-          __nanosleep(nap);
-          nap = min(nap * 2, 256u);
+    }
+    frozen = __syncthreads_or(frozen) != 0;
+    mbar_try(bar, it & 1);  // complete: each thread's own view of the copy's writes
+    const bool poisoned = tile == a.poison_col;  // test hook: the brick hands nothing over
+    if (!compute) {
+      t3_receive<T, G>(a, d, tile, d.epoch, box, x0, y0, zcnt, grp, &s_abort);
+      t3_next<G, OCT>(a, ntile, s_desc[(it + 1) & 1], &s_abort, wait_flag, wait_epoch);
+    } else {
+      // the planes of my column that update, one bit each in sweep order (inside
+      // the grid, in a visited block, not frozen).  Read once per brick, off the
+      // levels' dependency chain; most bricks freeze no node.
+      PlaneBits live = 0, changed = 0;
+      if (vxy) {
+        const unsigned mine = d.act >> ((gyl >> 3) * G::NBX + (gxl >> 3));
+#pragma unroll
+        for (int q = 0; q < NZB; ++q)
+          if ((mine >> (q * G::NBX * G::NBY)) & 1u) live |= PlaneBits(0xff) << (8 * q);
+        if (zcnt < BZ) live &= (PlaneBits(1) << zcnt) - 1;
+        if (frozen) {
+#pragma unroll 8
+          for (int p = 0; p < BZ; ++p) live &= ~(PlaneBits((smask[p * BY + gyl] >> (mshift + gxl)) & 1u) << p);
         }
+        if (szd < 0) live = G::flip(live);
       }
-    }
-    ok = __syncthreads_and(ok) != 0;
-    // the box copy has landed (bounded wait; on abort it is still drained below)
-    bool landed = mbar_wait(bar, par, a, tile, &s_abort);
-    if (!__syncthreads_and(ok && landed)) {
-      if (!landed && tid == 0) {  // let the copy land before the CTA leaves
-        const long long t0 = cycles();
-        while (!mbar_try(bar, par) && cycles() - t0 < 4000000000ll) {
-        }
-      }
-      break;
-    }
-    par ^= 1u;
-    // upwind halo faces: this sweep's values, written by the upwind bricks (L2)
-    if (li > 0) {  // x face
-      const int xu = sxd > 0 ? x0 - 1 : x0 + BX;
-      const int sxo = sxd > 0 ? 0 : BX + 1;
-      for (int q = tid; q < BZ * BY; q += G::NT) {
-        const int p = q / BY, r = q % BY;
-        if (p < zcnt && y0 + r <= ny)
-          box[(1 + p) * PL + (1 + r) * W + sxo] =
-              __ldcg(u + (long long)(z0 + p) * plane + (long long)(y0 + r) * px + xu);
-      }
-    }
-    if (lj > 0) {  // y face
-      const int yu = syd > 0 ? y0 - 1 : y0 + BY;
-      const int syo = syd > 0 ? 0 : BY + 1;
-      for (int q = tid; q < BZ * BX; q += G::NT) {
-        const int p = q / BX, xx = q % BX;
-        if (p < zcnt && x0 + xx <= nx)
-          box[(1 + p) * PL + syo * W + 1 + xx] =
-              __ldcg(u + (long long)(z0 + p) * plane + (long long)yu * px + x0 + xx);
-      }
-    }
-    if (lk > 0) {  // z face
-      const int zu = szd > 0 ? z0 - 1 : z0 + BZ;
-      const int szo = szd > 0 ? 0 : BZ + 1;
-      for (int q = tid; q < BY * BX; q += G::NT) {
-        const int r = q / BX, xx = q % BX;
-        if (y0 + r <= ny && x0 + xx <= nx)
-          box[szo * PL + (1 + r) * W + 1 + xx] =
-              __ldcg(u + (long long)zu * plane + (long long)(y0 + r) * px + x0 + xx);
-      }
-    }
-    __syncthreads();
-
-    // the levels: node (lx, ly, lz = L - lx - ly), sweep order
-    const int obase = (1 + gyl) * W + 1 + gxl + (szd > 0 ? PL : BZ * PL);  // lz = 0
-    const int dzo = szd > 0 ? PL : -PL;
-    T accb[NZB];
+      // replace-update: the smallest cap bound of my column in this brick
+      typename CB::type bnd = bnds[0];
 #pragma unroll
-    for (int q = 0; q < NZB; ++q) accb[q] = T(0);
-    const int lxy = lx + ly;
-    // pair-arithmetic rounds: the planes of my column that update, one bit per
-    // plane in sweep order (inside the grid, in an active 8^3 block, not
-    // frozen), read once per brick, off the levels' dependency chain (768^3
-    // polish round 22.0 -> 20.5 ms; the FP32 kernels were slower that way and
-    // test each node as they reach it)
-    constexpr bool kPlaneBits = OCT && ARITH == ARITH_PAIR;
-    using PlaneBits = typename std::conditional<(BZ > 32), unsigned long long, unsigned>::type;
-    PlaneBits live = 0;
-    if (kPlaneBits && vxy) {
-#pragma unroll 4
-      for (int lz = 0; lz < BZ; ++lz) {
-        const int gz = szd > 0 ? lz : BZ - 1 - lz;
-        bool on = gz < zcnt && ((actz >> (gz >> 3)) & 1u);
-        if (masked && on) on = !((smask[gz * BY + gyl] >> mshift) & 1u);
-        if (on) live |= PlaneBits(1) << lz;
+      for (int q = 1; q < NZB; ++q) bnd = CB::lower(bnd, bnds[q]);
+      // downwind faces: the planes whose x or y face node I send (every node of the
+      // face inside the grid: a reader takes those of visited blocks)
+      const bool mx = lx == BX - 1 && d.li < a.ntx - 1, my = ly == BY - 1 && d.lj < a.nty - 1;
+      PlaneBits face = 0;
+      if (vxy && !poisoned && (mx || my)) {
+        face = zcnt < BZ ? (PlaneBits(1) << zcnt) - 1 : PlaneBits(~0ull >> (64 - BZ));
+        if (szd < 0) face = G::flip(face);
       }
-    }
-    for (int L = lev0; L < lev1; ++L) {
-      const int lz = L - lxy;
-      if ((unsigned)lz < (unsigned)BZ) {
-        const int gz = szd > 0 ? lz : BZ - 1 - lz;
-        if (kPlaneBits ? ((live >> lz) & 1u) != 0 : (vxy && gz < zcnt)) {
-          const int o = obase + lz * dzo;
-          const T cv = box[o];
-          // the reference's minima keep grid orientation: min(u[x-1], u[x+1])
-          const T m0 = vmin<T, ARITH>(box[o - 1], box[o + 1]);
-          const T m1 = vmin<T, ARITH>(box[o - W], box[o + W]);
-          const T m2 = vmin<T, ARITH>(box[o - PL], box[o + PL]);
-          bool act = true;
-          if constexpr (!kPlaneBits) {
-            act = (actz >> (gz >> 3)) & 1u;
-            if (masked && act) act = !((smask[gz * BY + gyl] >> mshift) & 1u);
-          }
-          if (act) {
-            const T g = local_update<T, MODE, ARITH, ISO>(m0, m1, m2, k64, k32);
-            T nv;
-            if constexpr (MODE == MODE_REPLACE) {
-              typename CB::type b = bnd[0];
-#pragma unroll
-              for (int q = 1; q < NZB; ++q)
-                if ((gz >> 3) == q) b = bnd[q];
-              nv = CB::below(g, b) ? g : vmin<T, ARITH>(cap_value<T, ARITH>(capg + gbase + (long long)gz * plane), g);
-            } else {
-              nv = vmin<T, ARITH>(cv, g);
-            }
-            if (vdiffers<T, ARITH>(nv, cv)) {
-              box[o] = nv;
-              u[gbase + (long long)gz * plane] = nv;
-              const T d = node_change<T, ARITH>(cv, nv, hmin);
-              tmax = vmax_nonneg<T, ARITH>(tmax, d);
-              if (!OCT && blk_chg) {
-#pragma unroll
-                for (int q = 0; q < NZB; ++q)
-                  if ((gz >> 3) == q) accb[q] = vmax_nonneg<T, ARITH>(accb[q], d);
+      // mailbox entry of my face node of level L: row L - foff (the reader's level, wrapped)
+      const int foff = mx ? BX - 1 : BY - 1, fcol = mx ? G::MX + ly : G::MY + lx;
+      // the levels: node (lx, ly, lz = L - lx - ly), sweep order; live, face and
+      // changed planes as bits of 32-level words, bit L for the node of level L
+      const int dzo = szd > 0 ? PL : -PL;
+      T *p = box + (1 + gyl) * W + 1 + gxl + (szd > 0 ? PL : BZ * PL) + (d.lev0 - lxy) * dzo;  // my node of level L
+      T tmax = T(0);
+      const bool rec = !OCT && a.blk_chg != nullptr;
+      float acc = 0.0f;  // block-change output: my change in block accq of my column
+      int accq = 0;
+      const int accb = (gyl >> 3) * G::NBX + (gxl >> 3);
+      const int lev1 = d.lev1;
+      auto levels = [&](auto ftz) {
+#pragma unroll 1
+        for (int L = d.lev0; L < lev1;) {  // lev0 is a multiple of 8
+          const int c0 = L & ~31, cend = min(lev1, c0 + 32);
+          unsigned m = G::level_word(live, c0 - lxy) >> (L - c0), fm = G::level_word(face, c0 - lxy) >> (L - c0);
+          unsigned chgw = 0;
+#pragma unroll 1
+          for (; L < cend; L += G::GL, m >>= G::GL, fm >>= G::GL) {
+            // the faces of the next GL levels (the helper's waits are bounded, and end in an arrival)
+            if (tid < 32) {
+              while (!mbar_try(grp + L / G::GL, it & 1)) {
               }
             }
+            unsigned cg = 0;
+#pragma unroll(ARITH == ARITH_REF || (sizeof(T) == 8 && ARITH == ARITH_FAST) ? 1 : G::GL)
+            for (int i = 0; i < G::GL; ++i, p += dzo) {
+              level_bar<G::NC>();
+              const unsigned bit = 1u << i;
+              if (m & bit) {
+                const T v = *p;
+                // the reference's minima keep grid orientation: min(u[x-1], u[x+1])
+                const T m0 = vmin<T, ARITH>(p[-1], p[1]);
+                const T m1 = vmin<T, ARITH>(p[-W], p[W]);
+                const T m2 = vmin<T, ARITH>(p[-PL], p[PL]);
+                const T g = local_update<T, MODE, ARITH, ISO, decltype(ftz)::value>(m0, m1, m2, a.k64, a.k32);
+                T nv;
+                if constexpr (MODE == MODE_REPLACE) {
+                  nv = g;
+                  if (!CB::below(g, bnd)) {
+                    const int lz = L + i - lxy, gz = szd > 0 ? lz : BZ - 1 - lz;
+                    nv = vmin<T, ARITH>(cap_value<T, ARITH>(capg + (long long)(z0 + gz) * a.plane +
+                                                            (long long)(y0 + gyl) * a.px + (x0 + gxl)),
+                                        g);
+                  }
+                } else {
+                  nv = vmin<T, ARITH>(v, g);
+                }
+                if (vdiffers<T, ARITH>(nv, v)) {
+                  *p = nv;
+                  cg |= bit;
+                  T dv = T(0);
+                  if (rec || change_may_exceed<T, ARITH>(v, nv, a.hmin, tmax)) {
+                    dv = node_change<T, ARITH>(v, nv, a.hmin);
+                    tmax = vmax_nonneg<T, ARITH>(tmax, dv);
+                  }
+                  if (rec) {
+                    const int lz = L + i - lxy, q = (szd > 0 ? lz : BZ - 1 - lz) >> 3;
+                    if (q != accq) {
+                      if (acc > 0.0f) atomicMax(&s_chg[accq * (G::NBX * G::NBY) + accb], __float_as_uint(acc));
+                      accq = q;
+                      acc = 0.0f;
+                    }
+                    acc = fmaxf(acc, change_f<T, ARITH>(dv));
+                  }
+                }
+              }
+            }
+            if (fm & ((1u << G::GL) - 1u)) {  // the group's face nodes: the readers take them by groups too
+#pragma unroll
+              for (int i = 0; i < G::GL; ++i) {
+                if ((fm >> i) & 1u) {
+                  const T v = p[(i - G::GL) * dzo];
+                  int r = L + i - foff;
+                  if (r >= BZ) r -= BZ;
+                  mail_put<T>(d.mail + (r * (BX == BY || mx ? BY : BX) + fcol) * G::WV, v, d.epoch);
+                  if (mx && my) {  // the corner column: its y face too
+                    r = L + i - (BY - 1);
+                    if (r >= BZ) r -= BZ;
+                    mail_put<T>(d.mail + (G::MY + r * BX + lx) * G::WV, v, d.epoch);
+                  }
+                }
+              }
+            }
+            chgw |= cg << (L - c0);
           }
+          changed |= G::plane_bits(chgw, c0 - lxy);
         }
-      }
-      __syncthreads();
-    }
-    // per-block change: lanes of one warp with the same 8^3 block are lx in
-    // [0, 8) or [8, 16) of the warp's two rows (rounds record none)
-    if (!OCT && blk_chg) {
-#pragma unroll
-      for (int q = 0; q < NZB; ++q) {
-        T v = accb[q];
-#pragma unroll
-        for (int off = 1; off <= 16; off <<= 1) {
-          if (off == 8) continue;
-          const T w2 = __shfl_xor_sync(0xffffffffu, v, off);
-          v = vmax_nonneg<T, ARITH>(v, w2);
-        }
-        // only nodes inside the grid change, so v > 0 names a block of the grid
-        const int bz = bk * NZB + q;
-        if ((lane == 0 || lane == 8) && change_pos<T, ARITH>(v) && bz < a.nbz) {
-          const int bx = (x0 - 1 + gxl) >> 3, by = (y0 - 1 + gyl) >> 3;
-          atomicMax(blk_chg + ((long long)bz * a.nby + by) * a.nbx + bx, __float_as_uint(change_f<T, ARITH>(v)));
-        }
-      }
-    }
-    if constexpr (OCT) {  // this sweep's change word (one per sweep of the round)
-      T v = tmax;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v = vmax_nonneg<T, ARITH>(v, __shfl_xor_sync(0xffffffffu, v, off));
-      if (lane == 0 && change_pos<T, ARITH>(v)) {
-        if constexpr (sizeof(T) == 4)  // the low word of the sweep's 64-bit slot
-          atomicMax(reinterpret_cast<unsigned int *>(reinterpret_cast<unsigned long long *>(a.maxchg) + osw),
-                    __float_as_uint(v));
-        else
-          atomicMax(reinterpret_cast<unsigned long long *>(a.maxchg) + osw, change_u64<T, ARITH>(v));
-      }
-      tmax = T(0);
-    }
-    // publish: the barrier orders every thread's stores before thread 0's
-    // GPU-scope fence, which orders them before the flag
-    __syncthreads();
-    if (tid == 0 && tile != a.poison_col) publish_gpu(a.tflag + tile, epoch);
-  }
-  // the CTA's max change -> the grid's counter (one atomic per warp)
-  {
-    T v = tmax;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = vmax_nonneg<T, ARITH>(v, __shfl_xor_sync(0xffffffffu, v, off));
-    if (lane == 0 && change_pos<T, ARITH>(v)) {
-      if constexpr (sizeof(T) == 4)
-        atomicMax(reinterpret_cast<unsigned int *>(a.maxchg), __float_as_uint(v));
+      };
+      // the FP32 parts' roots flush subnormals unless the spacings can make one
+      constexpr bool kRoots32 = sizeof(T) == 4 || ARITH == ARITH_MIXED || ARITH == ARITH_PAIR;
+      if (!kRoots32 || a.k32.tiny)
+        levels(std::false_type{});
       else
-        atomicMax(reinterpret_cast<unsigned long long *>(a.maxchg), change_u64<T, ARITH>(v));
+        levels(std::true_type{});
+      // my z face node, the column's last
+      if (vxy && !poisoned && d.lk < a.ntz - 1)
+        mail_put<T>(d.mail + (G::MZ + (lxy % BY) * BX + lx) * G::WV,
+                    box[(1 + gyl) * W + 1 + gxl + (szd > 0 ? BZ : 1) * PL], d.epoch);
+      if (szd < 0) changed = G::flip(changed);
+      schgp[gyl * BX + gxl] = changed;
+      if (rec && acc > 0.0f) atomicMax(&s_chg[accq * (G::NBX * G::NBY) + accb], __float_as_uint(acc));
+      // the sweep's change word, per CTA
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1)
+        tmax = vmax_nonneg<T, ARITH>(tmax, __shfl_xor_sync(0xffffffffu, tmax, off));
+      if (lane == 0 && change_pos<T, ARITH>(tmax)) {
+        unsigned long long w;
+        if constexpr (sizeof(T) == 4)
+          w = __float_as_uint(tmax);
+        else
+          w = change_u64<T, ARITH>(tmax);
+        atomicMax(&s_max[OCT ? d.sweep : 0], w);
+      }
+    }
+    __syncthreads();  // the box holds the brick's new values
+    if (compute) {
+      // the rows with a changed node -> global memory, 32 / BX rows a warp
+      const int gx = tid % BX, gy = tid / BX;
+      PlaneBits row = schgp[tid], any;
+#pragma unroll
+      for (int off = 1; off < BX; off <<= 1) row |= __shfl_xor_sync(0xffffffffu, row, off);
+      any = row;
+#pragma unroll
+      for (int off = BX; off < 32; off <<= 1) any |= __shfl_xor_sync(0xffffffffu, any, off);
+      if (x0 + gx > a.nx || y0 + gy > a.ny) row = 0;
+      T *up = u + (long long)z0 * a.plane + (long long)(y0 + gy) * a.px + (x0 + gx);
+      const T *bp = box + PL + (1 + gy) * W + 1 + gx;
+      const long long pl = a.plane;
+#pragma unroll 1
+      for (int p = 0; any != 0; p += 4, any >>= 4, row >>= 4, bp += 4 * PL, up += 4 * pl) {
+        if ((any & 15u) == 0) continue;
+        T v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (row & (1u << i)) v[i] = bp[i * PL];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (row & (1u << i)) up[i * pl] = v[i];
+      }
+    }
+    fence_proxy_async();  // my accesses to the box come before the next copy's writes
+    if (__syncthreads_or(s_abort)) break;
+    // the brick is done: publish (a round's later sweeps wait for it).  The
+    // barrier orders every thread's stores before this thread's GPU-scope fence,
+    // which orders them before the flag.
+    if constexpr (OCT) {
+      if (tid == G::NC && !poisoned) publish_gpu(a.tflag + tile, d.epoch);
+    } else if (a.blk_chg != nullptr && tid < G::NB) {
+      // block changes: only nodes inside the grid change, so a positive one names a block of the grid
+      if (s_chg[tid]) {
+        const int bx = G::NBX * bi + tid % G::NBX, by = G::NBY * bj + (tid / G::NBX) % G::NBY;
+        const int bz = NZB * bk + tid / (G::NBX * G::NBY);
+        a.blk_chg[((long long)bz * a.nby + by) * a.nbx + bx] = s_chg[tid];
+        s_chg[tid] = 0;
+      }
+    }
+  }
+  // the CTA's change words -> the sweeps' counters
+  __syncthreads();
+  if (tid < (OCT ? 8 : 1) && s_max[tid]) {
+    if constexpr (OCT) {  // FP32: the low word of the sweep's 64-bit slot
+      atomicMax(reinterpret_cast<unsigned long long *>(a.maxchg) + tid, s_max[tid]);
+    } else if constexpr (sizeof(T) == 4) {
+      atomicMax(reinterpret_cast<unsigned int *>(a.maxchg), (unsigned)s_max[0]);
+    } else {
+      atomicMax(reinterpret_cast<unsigned long long *>(a.maxchg), s_max[0]);
     }
   }
 }
