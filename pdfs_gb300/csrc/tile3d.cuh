@@ -31,10 +31,12 @@
 // plus an L2 round trip per brick crossed.
 // Measured (octant rounds; FP32 full round / FP32 masked round / pair round): with
 // bricks that waited for whole upwind bricks, 768^3 22.0 / 13.0 / 20.5 ms, 320 x
-// 300 x 280 5.3 / 3.2 / 5.5 ms; handed over level by level, 23.6 / 9.5 / 16.7 and
-// 3.15 / 1.1 / 2.2 ms.  The 768^3 full round, which has bricks enough to fill the
-// chip, pays for the mail (issue slots are 56 % busy there); every grid with
-// fewer, and every masked round, gains.  Tried on the way: the helper stepping
+// 300 x 280 5.3 / 3.2 / 5.5 ms; handed over level by level, 22.1 / 8.5 / 15.1 and
+// 2.55 / 0.95 / 1.7 ms (23.6 / 9.5 / 16.7 and 3.15 / 1.1 / 2.2 while the helper
+// looked at the abort flag between its polls, tested every level's bits on its own
+// and z faces left at a brick's end).  The 768^3 full round, which has bricks
+// enough to fill the chip, gains nothing from the shorter chain (issue slots are
+// 56 % busy there).  Tried on the way: the helper stepping
 // through the levels' barrier (29.8 ms for the 768^3 full round), a second
 // helper warp sending the faces (27.9: 48 registers a thread, and the sender's
 // path was the level's), warps chained by mbarriers instead of a barrier a
@@ -366,53 +368,57 @@ __device__ __forceinline__ void t3_receive(const SweepArgs &a, const T3Desc &d, 
         nz |= LevelBits((1u << c8) - 1u) << (lane + (py ? 8 * q : BY - 8 * q - c8));
     }
   }
-  const int lev0 = d.lev0, lev1 = d.lev1;
   // past the last awaited level every level is ready
-  const int gend = min(lev1, __reduce_max_sync(0xffffffffu, max(G::top(nf), G::top(nz))));
+  const int gend = min(d.lev1, __reduce_max_sync(0xffffffffu, max(G::top(nf), G::top(nz))));
   // mail of level lv: row lv (mod the face's rows) of the upwind brick's face
   const long long upf = xf ? tile - d.sx : tile - d.sy * a.ntx, upz = tile - d.sz * a.ntx * a.nty;
   const unsigned long long *mf = a.pmail + (upf * G::MAIL + (xf ? G::MX : G::MY) + k) * G::WV;
   const unsigned long long *mz = a.pmail + (upz * G::MAIL + G::MZ + lane) * G::WV;
-  const int fcols = (xf ? BY : BX) * G::WV;
+  const int fcols = BX == BY ? BX * G::WV : (xf ? BY : BX) * G::WV;
   // box element read at level 0 and the step per level
   const int fs = pz ? PL : -PL, zs = py ? W : -W;
   T *bf = box + (pz ? 1 : BZ) * PL + (xf ? (1 + ku) * W + (px ? 0 : BX + 1) : (py ? 0 : BY + 1) * W + 1 + ku) - k * fs;
   T *bz = box + (pz ? 0 : BZ + 1) * PL + (py ? 1 : BY) * W + 1 + zu - lane * zs;
-  constexpr int SL = G::SL;
+  constexpr int GL = G::GL, SL = G::SL;
+  static_assert(BZ % GL == 0 && BY % GL == 0 && GL % SL == 0, "a group's rows are consecutive");
   bool live = true;  // false: gave up; the compute threads run out their levels (the call returns an error)
   for (int g = 0; g < G::NG; ++g) {
-    const int g0 = max(lev0, g * G::GL), g1 = min(gend, g * G::GL + G::GL);
-    for (int L = g0; L < g1 && live; L += SL) {
-      Mail<T> v[SL], w[SL];
-      const long long t_last = cycles();
-      unsigned nap = 0;
-      for (;;) {
-        bool ok = true;
+    if (g * GL < gend && live) {
+#pragma unroll 1
+      for (int L = g * GL; L < g * GL + GL; L += SL) {
+        const unsigned wf = (unsigned)(nf >> L) & ((1u << SL) - 1u);  // awaited: level L + i
+        const unsigned wz = L < BX + BY - 1 ? (unsigned)(nz >> L) & ((1u << SL) - 1u) : 0u;
+        const unsigned long long *pf = mf + (L >= BZ ? L - BZ : L) * fcols, *pzm = mz + (L % BY) * (BX * G::WV);
+        Mail<T> v[SL], w[SL];
+        const long long t_last = cycles();
+        unsigned nap = 0;
+        for (int tries = 0;; ++tries) {
 #pragma unroll
-        for (int i = 0; i < SL; ++i) {  // all the loads first: they are in flight together
-          const int lv = L + i;
-          if (lv < g1 && ((nf >> lv) & 1u)) v[i].load(mf + (lv >= BZ ? lv - BZ : lv) * fcols);
-          if (lv < g1 && ((nz >> lv) & 1u)) w[i].load(mz + (lv % BY) * (BX * G::WV));
+          for (int i = 0; i < SL; ++i) {  // all the loads first: they are in flight together
+            if (wf & (1u << i)) v[i].load(pf + i * fcols);
+            if (wz & (1u << i)) w[i].load(pzm + i * (BX * G::WV));
+          }
+          bool ok = true;
+#pragma unroll
+          for (int i = 0; i < SL; ++i) {
+            if (wf & (1u << i)) ok = ok && v[i].tagged(epoch);
+            if (wz & (1u << i)) ok = ok && w[i].tagged(epoch);
+          }
+          if (__all_sync(0xffffffffu, ok)) break;
+          // a poll is a round trip to L2: the first ones follow on one another (looking
+          // at the abort flag in between is another round trip on the sweep's chain)
+          if (tries >= 16 && helper_idle(a, tile, s_abort, t_last, nap)) {
+            live = false;
+            break;
+          }
         }
 #pragma unroll
         for (int i = 0; i < SL; ++i) {
-          const int lv = L + i;
-          if (lv < g1 && ((nf >> lv) & 1u)) ok = ok && v[i].tagged(epoch);
-          if (lv < g1 && ((nz >> lv) & 1u)) ok = ok && w[i].tagged(epoch);
+          if (wf & (1u << i)) bf[(L + i) * fs] = v[i].value();
+          if (wz & (1u << i)) bz[(L + i) * zs] = w[i].value();
         }
-        if (__all_sync(0xffffffffu, ok)) break;
-        if (helper_idle(a, tile, s_abort, t_last, nap)) {
-          live = false;
-          break;
-        }
+        __syncwarp();
       }
-#pragma unroll
-      for (int i = 0; i < SL; ++i) {
-        const int lv = L + i;
-        if (lv < g1 && ((nf >> lv) & 1u)) bf[lv * fs] = v[i].value();
-        if (lv < g1 && ((nz >> lv) & 1u)) bz[lv * zs] = w[i].value();
-      }
-      __syncwarp();
     }
     if (lane == 0) mbar_arrive(grp + g);
   }
@@ -567,6 +573,8 @@ __global__ void __launch_bounds__(T3Geo<T, BX_, BY_, BZ>::NT,
         face = zcnt < BZ ? (PlaneBits(1) << zcnt) - 1 : PlaneBits(~0ull >> (64 - BZ));
         if (szd < 0) face = G::flip(face);
       }
+      // my z face node, the column's last: its level, where a brick is downwind
+      const int zlev = vxy && !poisoned && d.lk < a.ntz - 1 ? lxy + BZ - 1 : -G::GL;
       // mailbox entry of my face node of level L: row L - foff (the reader's level, wrapped)
       const int foff = mx ? BX - 1 : BY - 1, fcol = mx ? G::MX + ly : G::MY + lx;
       // the levels: node (lx, ly, lz = L - lx - ly), sweep order; live, face and
@@ -636,6 +644,8 @@ __global__ void __launch_bounds__(T3Geo<T, BX_, BY_, BZ>::NT,
                 }
               }
             }
+            if ((unsigned)(zlev - L) < (unsigned)G::GL)
+              mail_put<T>(d.mail + (G::MZ + (lxy % BY) * BX + lx) * G::WV, p[(zlev - L - G::GL) * dzo], d.epoch);
             if (fm & ((1u << G::GL) - 1u)) {  // the group's face nodes: the readers take them by groups too
 #pragma unroll
               for (int i = 0; i < G::GL; ++i) {
@@ -663,10 +673,6 @@ __global__ void __launch_bounds__(T3Geo<T, BX_, BY_, BZ>::NT,
         levels(std::false_type{});
       else
         levels(std::true_type{});
-      // my z face node, the column's last
-      if (vxy && !poisoned && d.lk < a.ntz - 1)
-        mail_put<T>(d.mail + (G::MZ + (lxy % BY) * BX + lx) * G::WV,
-                    box[(1 + gyl) * W + 1 + gxl + (szd > 0 ? BZ : 1) * PL], d.epoch);
       if (szd < 0) changed = G::flip(changed);
       schgp[gyl * BX + gxl] = changed;
       if (rec && acc > 0.0f) atomicMax(&s_chg[accq * (G::NBX * G::NBY) + accb], __float_as_uint(acc));
