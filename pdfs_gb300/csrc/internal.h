@@ -78,6 +78,10 @@ cudaError_t launch_sweep(int which, int tile, int arith, bool iso, const SweepAr
 // a.torder / a.ntx.. / a.epoch filled in.
 cudaError_t launch_sweep_bricks(int which, int by, int bz, int arith, bool iso, const SweepArgs &a, const Layout &L,
                                 int sms, cudaStream_t st, int *grid_used);
+// One plain sweep (no block mask, no block-change output) on bricks of b x b x bz
+// (tile3d_plain.cu); a.torder / a.ntx.. / a.epoch filled in for them.
+cudaError_t launch_sweep_plain(int which, int b, int bz, int arith, bool iso, const SweepArgs &a, const Layout &L,
+                               int sms, cudaStream_t st, int *grid_used);
 // One unmasked sweep by the pencil kernel (pencil.cu): 16 x 16 pencils, the
 // column order / progress words of a 16 x 16 layout.
 cudaError_t launch_sweep_pencils(int which, int arith, bool iso, const SweepArgs &a, const Layout &L, int sms,
@@ -213,6 +217,11 @@ struct pdfs_ctx {
   uint8_t *tact = nullptr;
   int *tsparse = nullptr;
   int nt32[3] = {0, 0, 0}, nt64[3] = {0, 0, 0};
+  // pencil tiles: the bricks (b x b x bz) of their plain sweeps, or b = 0 for pencils
+  struct Plain {
+    int b = 0, bz = 0, nt[3] = {0, 0, 0};
+    int *tord = nullptr;
+  } plain32, plain64;
   int epoch = 0;  // flag value of the last brick or pencil sweep
   unsigned long long *pmail = nullptr;  // pencils: epoch-tagged face mailboxes
   int prow = 0;                          // their diagonals per face

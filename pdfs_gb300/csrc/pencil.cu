@@ -1,4 +1,5 @@
-// pencil.cu -- instantiations and launcher of the pencil sweep kernel (pencil.cuh).
+// pencil.cu -- instantiations and launcher of the pencil sweep kernel (pencil.cuh):
+// the FP64 sweeps that do not run on bricks (tile3d_plain.cu).
 #include <algorithm>
 
 #include "internal.h"
@@ -38,9 +39,7 @@ cudaError_t launch_sweep_pencils(int which, int arith, bool iso, const SweepArgs
   if (L.tx != 16 || L.ty != 16 || L.xo != 0 || a.blk_active || a.blk_chg || !a.pmail || a.prow < a.nz + 15 ||
       (which == 2 && (!a.bcap64 || !a.bcap32)))
     return cudaErrorInvalidValue;
-  if (which == 0)
-    return iso ? launch_pc<float, MODE_MIN, ARITH_FAST, true>(a, L, sms, st, g)
-               : launch_pc<float, MODE_MIN, ARITH_FAST, false>(a, L, sms, st, g);
+  if (which == 0) return cudaErrorInvalidValue;
   const bool rep = which == 2;
   switch (arith) {
     case ARITH_REF:

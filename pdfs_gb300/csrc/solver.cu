@@ -536,21 +536,42 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
   return PDFS_OK;
 }
 
-// Default tile choice (pdfs_autotune may override through opts.tile).
-// FP32: 16 x 16 pencils (tile 10: 3.6 ms per 768^3 sweep, against 3.9 ms for
-// 16 x 16 x 32 bricks and 7.9 ms for the best column tile); their masked
-// sweeps run on 16 x 16 x 32 bricks.
-// FP64: pencils (tile 6) for every arithmetic: 6.9 ms per 768^3 pair polish
-// sweep, against 8.1 ms for 16 x 16 x 16 bricks and 15.9 ms for mixed 32 x 6
-// columns; 51 ms per plain fast-arithmetic sweep against 55 ms for 32 x 4
-// columns (the reference arithmetic is even: both are FP64-pipe-bound).
-// The lane-column tiles (FP32 12/13, pairs 9/10) measured 6.1 / 3.7 ms per
-// FP32 sweep and 26.6 / 11.6 ms per pair polish sweep (8 / 4 rows): they stay
-// selectable (and autotuned), not the default.
+// Default tile choice (pdfs_autotune may override through opts.tile): the pencil
+// tiles, 10 (FP32) and 6 (FP64), whose masked and block-change-recording sweeps
+// run on bricks of 16 x 16 x 32 and 16 x 16 x 16.  The lane-column tiles (FP32
+// 12/13, pairs 9/10) measured 6.1 / 3.7 ms per 768^3 FP32 sweep and 26.6 / 11.6 ms
+// per pair polish sweep (8 / 4 rows): they stay selectable (and autotuned).
+//
+// Plain sweeps of the pencil tiles (no mask, no block changes), ms a sweep on
+// 64^3 / 251 x 233 x 241 / 384^3 / 1000 x 60 x 50 / 768^3 nodes:
+//   FP32: bricks of 16 x 16 x 32, 0.079 / 0.37 / 0.68 / 0.51 / 3.15, against 0.120 /
+//     0.52 / 1.04 / 0.71 / 3.94 on pencils.
+//   pairs and mixed: bricks of 16 x 16 x 32 up to 2^26 nodes, pencils above.  Pairs
+//     0.117 / 0.53 / 1.11 / 0.75 / 7.3, pencils 0.164 / 0.70 / 1.25 / 0.96 / 5.6; mixed
+//     0.175 / 0.83 / 1.71 / - / 9.8 and 0.214 / 1.00 / 1.79 / - / 8.5; both are even at
+//     448^3 (9.0e7 nodes: 1.57 and 1.63, 2.38 and 2.39).  A box of 64-bit values
+//     leaves room for two CTAs, and a brick reads its halo (27 % more bytes): what
+//     bricks save in the chain they lose once the chip is full.
+//   reference and fast: pencils.
+constexpr long long kPairBrickNodes = 1ll << 26;
+
 static void pick_tiles(pdfs_ctx *c) {
   const int t32 = c->o.tile & 0xff, t64 = (c->o.tile >> 8) & 0xff;
   c->t32 = t32 ? t32 : 10;
   c->t64 = t64 ? t64 : 6;
+  auto set = [&](pdfs_ctx::Plain &p, int b, int bz) {
+    p.b = b;
+    p.bz = bz;
+    p.nt[0] = (c->g.nx + b - 1) / b;
+    p.nt[1] = (c->g.ny + b - 1) / b;
+    p.nt[2] = (c->g.nz + bz - 1) / bz;
+  };
+  if (tile32(c->t32).pencil) set(c->plain32, 16, 32);
+  if (tile64(c->t64).pencil) {
+    if ((c->o.arith == PDFS_ARITH_MIXED || c->o.arith == PDFS_ARITH_PAIR) &&
+        (long long)c->g.nx * c->g.ny * c->g.nz <= kPairBrickNodes)
+      set(c->plain64, 16, 32);
+  }
 }
 
 extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_ctx **out) {
@@ -667,12 +688,22 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
     pmail_words = (size_t)((g->nx + 15) / 16) * ((g->ny + 15) / 16) * 2 * (size_t)c->prow * 16 * 2;
   }
   // bricks: three faces per brick (T3Geo::MAIL words, two per FP64 value)
+  auto brick_mail = [&](const int nt[3], int bx, int by, int bz, int words) {
+    pmail_words = std::max(pmail_words, (size_t)nt[0] * nt[1] * nt[2] * (size_t)(bz * by + bz * bx + bx * by) * words);
+  };
+  std::vector<int> bp[2];  // ticket orders of the pencil tiles' plain sweeps
   for (int k = 0; k < 2; ++k) {
     const TileShape ts = k ? s64 : s32;
     const int *nt = k ? c->nt64 : c->nt32;
-    if (ts.bz == 0 || o.precision == (k ? PDFS_PREC_FP32 : PDFS_PREC_FP64)) continue;
-    pmail_words = std::max(pmail_words, (size_t)nt[0] * nt[1] * nt[2] *
-                                            (size_t)(ts.bz * ts.ty + ts.bz * ts.tx + ts.tx * ts.ty) * (k ? 2 : 1));
+    pdfs_ctx::Plain &p = k ? c->plain64 : c->plain32;
+    if (o.precision == (k ? PDFS_PREC_FP32 : PDFS_PREC_FP64)) {
+      p.b = 0;
+      continue;
+    }
+    if (ts.bz) brick_mail(nt, ts.tx, ts.ty, ts.bz, k ? 2 : 1);
+    if (!p.b) continue;
+    brick_mail(p.nt, p.b, p.b, p.bz, k ? 2 : 1);
+    if (p.b != ts.tx || p.bz != ts.bz) bp[k] = brick_order(p.nt[0], p.nt[1], p.nt[2]);
   }
   std::vector<std::pair<void **, size_t>> plan;
   auto want = [&](auto **p, size_t bytes) {
@@ -708,6 +739,8 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
   }
   want(&c->tord32, bo[0].size() * 4);
   want(&c->tord64, bo[1].size() * 4);
+  want(&c->plain32.tord, bp[0].size() * 4);
+  want(&c->plain64.tord, bp[1].size() * 4);
   want(&c->tflag, nflags * 4);
   want(&c->tact, nflags);
   want(&c->tsparse, nflags ? (nflags + 1) * 4 : 0);
@@ -739,6 +772,13 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
     if (!bo[k].empty() &&
         (e = cudaMemcpyAsync(dst, bo[k].data(), bo[k].size() * 4, cudaMemcpyHostToDevice, c->st)) != cudaSuccess)
       return fail(e);
+  }
+  for (int k = 0; k < 2; ++k) {
+    pdfs_ctx::Plain &p = k ? c->plain64 : c->plain32;
+    if (!bp[k].empty() &&
+        (e = cudaMemcpyAsync(p.tord, bp[k].data(), bp[k].size() * 4, cudaMemcpyHostToDevice, c->st)) != cudaSuccess)
+      return fail(e);
+    if (p.b && bp[k].empty()) p.tord = k ? c->tord64 : c->tord32;  // the masked sweeps' bricks
   }
   if (nflags && (e = cudaMemsetAsync(c->tflag, 0, nflags * 4, c->st)) != cudaSuccess) return fail(e);
   if (pmail_words && (e = cudaMemsetAsync(c->pmail, 0, pmail_words * 8, c->st)) != cudaSuccess) return fail(e);
@@ -1103,7 +1143,8 @@ static int run_sweep(pdfs_ctx *c, int which, int sn, const uint8_t *active, unsi
   // (pencils that recorded block changes measured no faster: 37.4 against 36.9 ms
   // for the 8 recording sweeps of the 768^3 headline solve)
   const bool pencil = ts.pencil && !active && !blk_chg;
-  if (ts.bz == 0 || pencil) CK(cudaMemsetAsync(c->progress, 0, (size_t)L.ncx * L.ncy * L.ty * 4, c->st));
+  const pdfs_ctx::Plain &pl = f32 ? c->plain32 : c->plain64;
+  if (ts.bz == 0 || (pencil && !pl.b)) CK(cudaMemsetAsync(c->progress, 0, (size_t)L.ncx * L.ncy * L.ty * 4, c->st));
   CK(cudaMemsetAsync(c->dstat, 0, offsetof(DevStatus, active_blocks), c->st));
   if (blk_chg) CK(cudaMemsetAsync(blk_chg, 0, (size_t)c->nblocks * 4, c->st));
   CK(cudaMemsetAsync(c->ticket, 0, 4, c->st));
@@ -1113,7 +1154,14 @@ static int run_sweep(pdfs_ctx *c, int which, int sn, const uint8_t *active, unsi
                                                        : ARITH_FAST;
   int grid = 0;
   CK(cudaEventRecord(c->k0, c->st));
-  if (pencil) {
+  if (pencil && pl.b) {
+    a.epoch = ++c->epoch;  // mailbox words of every earlier sweep carry a smaller tag
+    a.torder = pl.tord;
+    a.ntx = pl.nt[0];
+    a.nty = pl.nt[1];
+    a.ntz = pl.nt[2];
+    CK(launch_sweep_plain(which, pl.b, pl.bz, arith, iso, a, L, c->sms, c->st, &grid));
+  } else if (pencil) {
     a.epoch = ++c->epoch;  // mailbox words of every earlier sweep carry a smaller tag
     CK(launch_sweep_pencils(which, arith, iso, a, L, c->sms, c->st, &grid));
   } else if (ts.bz > 0) {

@@ -1,8 +1,7 @@
 // tile3d.cu -- instantiations and launcher of the brick sweep kernel (tile3d.cuh).
 #include <algorithm>
 
-#include "internal.h"
-#include "tile3d.cuh"
+#include "tile3d_launch.cuh"
 
 namespace pdfs {
 
@@ -25,51 +24,29 @@ std::vector<int> brick_order(int ntx, int nty, int ntz) {
   return o;
 }
 
-template <class T, int BY, int BZ, int MODE, int ARITH, bool ISO>
-static cudaError_t launch_t3(const SweepArgs &a, const Layout &L, int sms, cudaStream_t st, int *grid_used) {
-  using G = T3Geo<T, 16, BY, BZ>;
-  auto kern = t3_sweep_kernel<T, 16, BY, BZ, MODE, ARITH, ISO>;
-  CUtensorMap m;
-  cudaError_t e = encode_field_map(&m, a.u, sizeof(T), L, a.nz + 2, G::W, G::RY, G::RZ);
-  if (e != cudaSuccess) return e;
-  const size_t smem = G::BYTES;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, G::NT, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  const int ntile = a.ntx * a.nty * a.ntz;
-  int grid = std::min(per_sm * sms, ntile);
-  if (grid < 1) grid = 1;
-  kern<<<grid, G::NT, smem, st>>>(m, a);
-  if (grid_used) *grid_used = grid;
-  return cudaGetLastError();
-}
-
 template <int BY, int BZ>
 static cudaError_t dispatch_t3(int which, int arith, bool iso, const SweepArgs &a, const Layout &L, int sms,
                                cudaStream_t st, int *g) {
   if (which == 0)
-    return iso ? launch_t3<float, BY, BZ, MODE_MIN, ARITH_FAST, true>(a, L, sms, st, g)
-               : launch_t3<float, BY, BZ, MODE_MIN, ARITH_FAST, false>(a, L, sms, st, g);
+    return iso ? launch_t3<float, 16, BY, BZ, MODE_MIN, ARITH_FAST, true, false>(a, L, sms, st, g)
+               : launch_t3<float, 16, BY, BZ, MODE_MIN, ARITH_FAST, false, false>(a, L, sms, st, g);
   {
     if (which == 1) {
-      if (arith == ARITH_REF) return launch_t3<double, BY, BZ, MODE_MIN, ARITH_REF, false>(a, L, sms, st, g);
-      if (arith == ARITH_FAST) return launch_t3<double, BY, BZ, MODE_MIN, ARITH_FAST, false>(a, L, sms, st, g);
+      if (arith == ARITH_REF) return launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_REF, false, false>(a, L, sms, st, g);
+      if (arith == ARITH_FAST) return launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_FAST, false, false>(a, L, sms, st, g);
       if (arith == ARITH_PAIR)
-        return iso ? launch_t3<double, BY, BZ, MODE_MIN, ARITH_PAIR, true>(a, L, sms, st, g)
-                   : launch_t3<double, BY, BZ, MODE_MIN, ARITH_PAIR, false>(a, L, sms, st, g);
-      return iso ? launch_t3<double, BY, BZ, MODE_MIN, ARITH_MIXED, true>(a, L, sms, st, g)
-                 : launch_t3<double, BY, BZ, MODE_MIN, ARITH_MIXED, false>(a, L, sms, st, g);
+        return iso ? launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_PAIR, true, false>(a, L, sms, st, g)
+                   : launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_PAIR, false, false>(a, L, sms, st, g);
+      return iso ? launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_MIXED, true, false>(a, L, sms, st, g)
+                 : launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_MIXED, false, false>(a, L, sms, st, g);
     }
-    if (arith == ARITH_REF) return launch_t3<double, BY, BZ, MODE_REPLACE, ARITH_REF, false>(a, L, sms, st, g);
-    if (arith == ARITH_FAST) return launch_t3<double, BY, BZ, MODE_REPLACE, ARITH_FAST, false>(a, L, sms, st, g);
+    if (arith == ARITH_REF) return launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_REF, false, false>(a, L, sms, st, g);
+    if (arith == ARITH_FAST) return launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_FAST, false, false>(a, L, sms, st, g);
     if (arith == ARITH_PAIR)
-      return iso ? launch_t3<double, BY, BZ, MODE_REPLACE, ARITH_PAIR, true>(a, L, sms, st, g)
-                 : launch_t3<double, BY, BZ, MODE_REPLACE, ARITH_PAIR, false>(a, L, sms, st, g);
-    return iso ? launch_t3<double, BY, BZ, MODE_REPLACE, ARITH_MIXED, true>(a, L, sms, st, g)
-               : launch_t3<double, BY, BZ, MODE_REPLACE, ARITH_MIXED, false>(a, L, sms, st, g);
+      return iso ? launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_PAIR, true, false>(a, L, sms, st, g)
+                 : launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_PAIR, false, false>(a, L, sms, st, g);
+    return iso ? launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_MIXED, true, false>(a, L, sms, st, g)
+               : launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_MIXED, false, false>(a, L, sms, st, g);
   }
 }
 
@@ -269,23 +246,7 @@ int octant_scratch_ints(int ntx, int nty, int ntz) {
 
 template <class T, int BZ, int MODE, int ARITH, bool ISO>
 static cudaError_t launch_oct(const SweepArgs &a, const Layout &L, int sms, cudaStream_t st, int *grid_used) {
-  using G = T3Geo<T, 16, 16, BZ>;
-  auto kern = t3_sweep_kernel<T, 16, 16, BZ, MODE, ARITH, ISO, true>;
-  CUtensorMap m;
-  cudaError_t e = encode_field_map(&m, a.u, sizeof(T), L, a.nz + 2, G::W, G::RY, G::RZ);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::BYTES);
-  if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, G::NT, G::BYTES);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  // every CTA resident: a ticket waits only on smaller tickets
-  int grid = std::min(per_sm * sms, kOctMax * a.ntx * a.nty * a.ntz);
-  if (grid < 1) grid = 1;
-  kern<<<grid, G::NT, G::BYTES, st>>>(m, a);
-  if (grid_used) *grid_used = grid;
-  return cudaGetLastError();
+  return launch_t3<T, 16, 16, BZ, MODE, ARITH, ISO, true>(a, L, sms, st, grid_used);
 }
 
 cudaError_t launch_octant_round(int which, int arith, bool iso, int nsw, const SweepArgs &a0, const Layout &L,
@@ -378,8 +339,8 @@ cudaError_t launch_sweep_bricks(int which, int by, int bz, int arith, bool iso, 
   if (by == 16 && bz == 32) return dispatch_t3<16, 32>(which, arith, iso, a, L, sms, st, g);
   if (by == 8 && bz == 32) return dispatch_t3<8, 32>(which, arith, iso, a, L, sms, st, g);
   if (by == 8 && bz == 48 && which == 0)  // FP32 only
-    return iso ? launch_t3<float, 8, 48, MODE_MIN, ARITH_FAST, true>(a, L, sms, st, g)
-               : launch_t3<float, 8, 48, MODE_MIN, ARITH_FAST, false>(a, L, sms, st, g);
+    return iso ? launch_t3<float, 16, 8, 48, MODE_MIN, ARITH_FAST, true, false>(a, L, sms, st, g)
+               : launch_t3<float, 16, 8, 48, MODE_MIN, ARITH_FAST, false, false>(a, L, sms, st, g);
   return cudaErrorInvalidValue;
 }
 

@@ -717,11 +717,11 @@ __global__ void __launch_bounds__(T3Geo<T, BX_, BY_, BZ>::NT,
     }
     fence_proxy_async();  // my accesses to the box come before the next copy's writes
     if (__syncthreads_or(s_abort)) break;
-    // the brick is done: publish (a round's later sweeps wait for it).  The
+    // the brick is done: publish (a round's later sweeps, if any, wait for it).  The
     // barrier orders every thread's stores before this thread's GPU-scope fence,
     // which orders them before the flag.
     if constexpr (OCT) {
-      if (tid == G::NC && !poisoned) publish_gpu(a.tflag + tile, d.epoch);
+      if (tid == G::NC && !poisoned && a.tflag) publish_gpu(a.tflag + tile, d.epoch);
     } else if (a.blk_chg != nullptr && tid < G::NB) {
       // block changes: only nodes inside the grid change, so a positive one names a block of the grid
       if (s_chg[tid]) {
