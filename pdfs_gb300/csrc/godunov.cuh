@@ -30,6 +30,21 @@ __device__ __forceinline__ void cswap(T &a, T &b) {
   b = t;
 }
 
+// What god64.cuh needs of the spacings for one sorted order (0, 1, 2) of the
+// axes' minima: d spacings, q = d^2, w = 1/d^2, and their combinations, each
+// rounded as the expressions of god_ref64 round them.
+struct GodPerm64 {
+  double d0, q0, q1, q2;
+  double d01, d012;      // d0 d1, (d0 d1) d2
+  double s, is;          // q0 + q1, 1 / s
+  double q01, q02, q12;  // q0 q1, q0 q2, q1 q2
+  double den, iden;      // (q0 q1 + q0 q2) + q1 q2, 1 / den
+  double w1, w2, w01;    // w0 w1
+  double ws, iws;        // w0 + w1, 1 / ws
+  double wsum, iwsum;    // w of all axes, 1 / wsum
+  double pad;            // rows of 21 doubles: six of them read at once share no bank
+};
+
 // Per-sweep constants of the local solver.
 struct GodConst64 {
   double h[3];   // spacings

@@ -239,6 +239,7 @@ struct pdfs_ctx {
   unsigned int *bchg = nullptr;  // [kRing][nblocks] float bits of per-block max change, rotating
   uint8_t *bact = nullptr;       // [nblocks] active mask of the next sweep
   uint8_t *omask = nullptr;      // [nblocks] polish: the orderings that matter to each block
+  pdfs::GodPerm64 *kperm = nullptr;  // FP64 solvers' constants by sorted axis order (god64.cuh)
   int *toct = nullptr;           // octant rounds: [8][bricks] tickets, 17 counts / offsets, the merged
                                  // ticket list and its plan (octant_scratch_ints)
   bool oct32_ok = false, oct64_ok = false;  // octant rounds available (FP32 / polish brick shapes)

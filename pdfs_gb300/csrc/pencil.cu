@@ -1,5 +1,6 @@
 // pencil.cu -- instantiations and launcher of the pencil sweep kernel (pencil.cuh):
-// the FP64 sweeps that do not run on bricks (tile3d_plain.cu).
+// the FP32-pair and mixed sweeps of large grids.  Every other plain sweep of the
+// pencil tiles runs on bricks (tile3d_plain.cu).
 #include <algorithm>
 
 #include "internal.h"
@@ -42,12 +43,6 @@ cudaError_t launch_sweep_pencils(int which, int arith, bool iso, const SweepArgs
   if (which == 0) return cudaErrorInvalidValue;
   const bool rep = which == 2;
   switch (arith) {
-    case ARITH_REF:
-      return rep ? launch_pc<double, MODE_REPLACE, ARITH_REF, false>(a, L, sms, st, g)
-                 : launch_pc<double, MODE_MIN, ARITH_REF, false>(a, L, sms, st, g);
-    case ARITH_FAST:
-      return rep ? launch_pc<double, MODE_REPLACE, ARITH_FAST, false>(a, L, sms, st, g)
-                 : launch_pc<double, MODE_MIN, ARITH_FAST, false>(a, L, sms, st, g);
     case ARITH_MIXED:
       if (iso)
         return rep ? launch_pc<double, MODE_REPLACE, ARITH_MIXED, true>(a, L, sms, st, g)

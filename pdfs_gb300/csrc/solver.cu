@@ -387,6 +387,44 @@ extern "C" const char *pdfs_status_string(int s) {
 
 extern "C" const char *pdfs_version(void) { return "pdfs-gb300 0.1 (sm_103a)"; }
 
+// The constants of god64.cuh for the six sorted orders of the axes (index 2 a0
+// + (a1 > a2)).  Every operation is rounded on its own (volatile: no contraction
+// into a multiply-add on the host), as the device's expressions round.
+static void fill_perm(const pdfs_grid &g, GodPerm64 out[6]) {
+  const double h[3] = {g.dx, g.dy, g.dz};
+  auto mul = [](double a, double b) { volatile double r = a * b; return (double)r; };
+  auto add = [](double a, double b) { volatile double r = a + b; return (double)r; };
+  double wsum = 0.0;
+  for (int i = 0; i < 3; ++i) wsum = add(wsum, 1.0 / mul(h[i], h[i]));
+  for (int a0 = 0; a0 < 3; ++a0)
+    for (int swap = 0; swap < 2; ++swap) {
+      const int lo = a0 == 0 ? 1 : 0, hi = a0 == 2 ? 1 : 2, a1 = swap ? hi : lo, a2 = swap ? lo : hi;
+      GodPerm64 &p = out[2 * a0 + swap];
+      const double d0 = h[a0], d1 = h[a1], d2 = h[a2];
+      p.d0 = d0;
+      p.q0 = mul(d0, d0);
+      p.q1 = mul(d1, d1);
+      p.q2 = mul(d2, d2);
+      p.d01 = mul(d0, d1);
+      p.d012 = mul(p.d01, d2);
+      p.s = add(p.q0, p.q1);
+      p.is = 1.0 / p.s;
+      p.q01 = mul(p.q0, p.q1);
+      p.q02 = mul(p.q0, p.q2);
+      p.q12 = mul(p.q1, p.q2);
+      p.den = add(add(p.q01, p.q02), p.q12);
+      p.iden = 1.0 / p.den;
+      const double w0 = 1.0 / p.q0;
+      p.w1 = 1.0 / p.q1;
+      p.w2 = 1.0 / p.q2;
+      p.w01 = mul(w0, p.w1);
+      p.ws = add(w0, p.w1);
+      p.iws = 1.0 / p.ws;
+      p.wsum = wsum;
+      p.iwsum = 1.0 / wsum;
+    }
+}
+
 // Context blocks (the arena of a context's buffers, the transfer stage) are
 // kept in a per-process cache when a context is destroyed, up to a quarter of
 // the device's memory, and handed to the next context that needs a block of
@@ -552,7 +590,12 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 //     448^3 (9.0e7 nodes: 1.57 and 1.63, 2.38 and 2.39).  A box of 64-bit values
 //     leaves room for two CTAs, and a brick reads its halo (27 % more bytes): what
 //     bricks save in the chain they lose once the chip is full.
-//   reference and fast: pencils.
+//   reference and fast: bricks of 8 x 8 x 16 with the solvers of god64.cuh.
+//     Reference 0.54 / 3.7 / 10.1 / 3.6 / -, pencils 1.35 / 10.5 / 18.7 / - / -; fast
+//     0.29 / 1.7 / 4.6 / 1.8 / -, pencils 0.82 / 5.6 / 10.4 / - / -.  A level costs one
+//     warp some 60 (25) FP64 operations of 64 cycles each however few of its lanes
+//     hold a node, so small faces, which lag their upwind bricks by fewer levels, win:
+//     16 x 16 x 16 bricks take 0.73 / 4.5 / 10.6 and 0.36 / 2.0 / 5.0.
 constexpr long long kPairBrickNodes = 1ll << 26;
 
 static void pick_tiles(pdfs_ctx *c) {
@@ -568,8 +611,9 @@ static void pick_tiles(pdfs_ctx *c) {
   };
   if (tile32(c->t32).pencil) set(c->plain32, 16, 32);
   if (tile64(c->t64).pencil) {
-    if ((c->o.arith == PDFS_ARITH_MIXED || c->o.arith == PDFS_ARITH_PAIR) &&
-        (long long)c->g.nx * c->g.ny * c->g.nz <= kPairBrickNodes)
+    if (c->o.arith == PDFS_ARITH_REFERENCE || c->o.arith == PDFS_ARITH_FAST)
+      set(c->plain64, 8, 16);
+    else if ((long long)c->g.nx * c->g.ny * c->g.nz <= kPairBrickNodes)
       set(c->plain64, 16, 32);
   }
 }
@@ -721,6 +765,7 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
   want(&c->progress, c->progress_ints * 4);
   want(&c->mailbox, c->mailbox_bytes);
   want(&c->ticket, 16);
+  want(&c->kperm, 6 * sizeof(GodPerm64));
   want(&c->dstat, sizeof(DevStatus));
   want(&c->bchg, (size_t)c->nblocks * kRing * 4);
   want(&c->bact, (size_t)c->nblocks);
@@ -764,6 +809,9 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
   }
   mark("allocation");
   if ((e = cudaHostAlloc(&c->hstat, sizeof(DevStatus), cudaHostAllocDefault)) != cudaSuccess) return fail(e);
+  GodPerm64 perm[6];
+  fill_perm(*g, perm);
+  if ((e = cudaMemcpyAsync(c->kperm, perm, sizeof perm, cudaMemcpyHostToDevice, c->st)) != cudaSuccess) return fail(e);
   if (!wb.empty() &&
       (e = cudaMemcpyAsync(c->mlp_w, wb.data(), PDFS_MLP_PARAMS * 2, cudaMemcpyHostToDevice, c->st)) != cudaSuccess)
     return fail(e);
@@ -1026,6 +1074,8 @@ void pdfs::fill_sweep_args(const pdfs_ctx *c, int which, int sn, const uint8_t *
   a.epoch = c->epoch;
   a.pmail = c->pmail;
   a.prow = c->prow;
+  a.kperm = std::min(g.dx, std::min(g.dy, g.dz)) >= 1e-30 && std::max(g.dx, std::max(g.dy, g.dz)) <= 1e30 ? c->kperm
+                                                                                                              : nullptr;
   long long wait_ms = c->o.spin_limit > 0 ? c->o.spin_limit : 4000;
   if (getenv("PDFS_WAIT_MS")) wait_ms = atoll(getenv("PDFS_WAIT_MS"));
   a.wait_cycles = wait_ms * 1000000LL * 21 / 10;  // at most 2.07 GHz: never shorter than wait_ms

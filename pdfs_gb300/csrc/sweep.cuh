@@ -117,6 +117,10 @@ struct SweepArgs {
   unsigned oct_full;
   const uint8_t *oct_bits;
   const uint8_t *oct_tbits;
+  // FP64 reference and fast arithmetic on bricks (god64.cuh): by the sorted
+  // order of the axes' minima (sort64's index), in device memory; nullptr for
+  // spacings outside 1e-30 .. 1e30 (the plain solvers then)
+  const GodPerm64 *kperm;
 };
 
 // Arguments of the lane-column sweep (lanecol.cuh).

@@ -55,11 +55,12 @@
 // records DEV_ERR_TIMEOUT, raises the abort flag, lets its own TMA copy land
 // and returns.
 #pragma once
+#include "god64.cuh"
 #include "sweep.cuh"
 
 namespace pdfs {
 
-template <class T, int BX_, int BY_, int BZ>
+template <class T, int BX_, int BY_, int BZ, int GL_ = 4>
 struct T3Geo {
   static constexpr int BX = BX_, BY = BY_;
   // box row: x0-1 .. x0+BX, rounded up to 16 bytes; the field's index has no
@@ -76,7 +77,8 @@ struct T3Geo {
   // z face [(lx + ly) % BY][lx] -- one row per level of the reading brick, and
   // (the modulus) no unused entries
   static constexpr int MX = 0, MY = BZ * BY, MZ = MY + BZ * BX, MAIL = MZ + BX * BY;
-  static constexpr int SL = sizeof(T) == 4 ? 4 : 2;  // levels polled at a time
+  static constexpr int GL = GL_;  // levels handed over together
+  static constexpr int SL = GL < (sizeof(T) == 4 ? 4 : 2) ? GL : sizeof(T) == 4 ? 4 : 2;  // levels polled at a time
   static constexpr int NBX = BX / 8, NBY = BY / 8, NZB = BZ / 8;  // 8^3 scheduler blocks per brick
   static constexpr int NB = NBX * NBY * NZB;
   static constexpr unsigned BOX_BYTES = (unsigned)(W * RY * RZ * sizeof(T));
@@ -85,7 +87,7 @@ struct T3Geo {
   static constexpr size_t OFF_CHG = OFF_MASK + (size_t)BZ * BY * 4;
   static constexpr size_t OFF_BAR = OFF_CHG + (size_t)NC * sizeof(PlaneBits);
   // the box's barrier, then one per GL levels (their upwind faces are there)
-  static constexpr int GL = 4, NG = (NL + GL - 1) / GL;
+  static constexpr int NG = (NL + GL - 1) / GL;
   static constexpr size_t BYTES = OFF_BAR + 8 + (size_t)NG * 8;
   // resident CTAs asked of the compiler: what shared memory allows, at most 4
   // (56 registers a thread: 3 CTAs with more cost the 768^3 rounds 4 to 9 %)
@@ -120,6 +122,18 @@ struct T3Geo {
   static_assert(BX + BY <= 32 && NB <= 32 && NZB * (NBX + NBY) + NBX * NBY <= 32, "one lane each");
   static_assert((W * sizeof(T)) % 16 == 0, "TMA rows are 16-byte multiples");
 };
+
+// FP64 reference and fast arithmetic: the solvers of god64.cuh.
+template <class T, int ARITH>
+constexpr bool kGod64Of = sizeof(T) == 8 && (ARITH == ARITH_REF || ARITH == ARITH_FAST);
+
+// Their faces go over after every level (64^3 / 384^3 reference sweeps in 8 x 8 x 16
+// bricks, all else equal: 953 us and 12.2 ms; in groups of 2, 1128 and 12.9; of 4,
+// 1292 and 13.4): a level is 2000 to 4000 cycles, more than an L2 round trip.  An
+// FP32 or pair level is 200 to 300: groups of 4 (of 2: 7 to 15 % faster on FP32
+// grids to 64^3, 7 % slower at 768^3 and for pairs).
+template <class T, int BX, int BY, int BZ, int ARITH>
+using T3GeoOf = T3Geo<T, BX, BY, BZ, kGod64Of<T, ARITH> ? 1 : 4>;
 
 // The levels' barrier: the compute threads.
 template <int N>
@@ -435,10 +449,10 @@ __device__ __forceinline__ void t3_receive(const SweepArgs &a, const T3Desc &d, 
 // after the ones it waits on, so every wait is on a smaller ticket.  The
 // result is the sequential sweeps', bit for bit.
 template <class T, int BX_, int BY_, int BZ, int MODE, int ARITH, bool ISO, bool OCT = false>
-__global__ void __launch_bounds__(T3Geo<T, BX_, BY_, BZ>::NT,
-                                  (sizeof(T) == 4 || ARITH == ARITH_PAIR) ? T3Geo<T, BX_, BY_, BZ>::CTAS : 2)
+__global__ void __launch_bounds__(T3GeoOf<T, BX_, BY_, BZ, ARITH>::NT,
+                                  (sizeof(T) == 4 || ARITH == ARITH_PAIR) ? T3GeoOf<T, BX_, BY_, BZ, ARITH>::CTAS : 2)
     t3_sweep_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ SweepArgs a) {
-  using G = T3Geo<T, BX_, BY_, BZ>;
+  using G = T3GeoOf<T, BX_, BY_, BZ, ARITH>;
   using PlaneBits = typename G::PlaneBits;
   constexpr int BX = G::BX, BY = G::BY, W = G::W, PL = G::PL, NZB = G::NZB;
   extern __shared__ __align__(1024) unsigned char sm[];
@@ -471,6 +485,13 @@ __global__ void __launch_bounds__(T3Geo<T, BX_, BY_, BZ>::NT,
     mbar_init(bar, 1);
     for (int g = 0; g < G::NG; ++g) mbar_init(grp + g, 1);
     mbar_fence_init();
+  }
+  // FP64 reference and fast arithmetic: the spacings' constants by sorted order
+  constexpr bool kGod64 = kGod64Of<T, ARITH>;
+  __shared__ GodPerm64 s_perm[kGod64 ? 6 : 1];
+  if (kGod64 && a.kperm) {
+    for (int q = tid; q < (int)(6 * sizeof(GodPerm64) / 8); q += G::NT)
+      reinterpret_cast<double *>(s_perm)[q] = reinterpret_cast<const double *>(a.kperm)[q];
   }
   __shared__ uint8_t s_col[G::NC];  // diagonal order -> ly * BX + lx
   if (compute) s_col[diag_rank<BX, BY>(tid % BX, tid / BX)] = (uint8_t)tid;
@@ -601,36 +622,41 @@ __global__ void __launch_bounds__(T3Geo<T, BX_, BY_, BZ>::NT,
               }
             }
             unsigned cg = 0;
-#pragma unroll(ARITH == ARITH_REF || (sizeof(T) == 8 && ARITH == ARITH_FAST) ? 1 : G::GL)
+#pragma unroll
             for (int i = 0; i < G::GL; ++i, p += dzo) {
               level_bar<G::NC>();
               const unsigned bit = 1u << i;
               if (m & bit) {
                 const T v = *p;
-                // the reference's minima keep grid orientation: min(u[x-1], u[x+1])
-                const T m0 = vmin<T, ARITH>(p[-1], p[1]);
-                const T m1 = vmin<T, ARITH>(p[-W], p[W]);
-                const T m2 = vmin<T, ARITH>(p[-PL], p[PL]);
-                const T g = local_update<T, MODE, ARITH, ISO, decltype(ftz)::value>(m0, m1, m2, a.k64, a.k32);
+                T g;
+                if constexpr (kGod64) {
+                  g = god64_node<ARITH>(p[-1], p[1], p[-W], p[W], p[-PL], p[PL], a.k64, a.kperm ? s_perm : nullptr);
+                } else {
+                  // the reference's minima keep grid orientation: min(u[x-1], u[x+1])
+                  const T m0 = vmin<T, ARITH>(p[-1], p[1]);
+                  const T m1 = vmin<T, ARITH>(p[-W], p[W]);
+                  const T m2 = vmin<T, ARITH>(p[-PL], p[PL]);
+                  g = local_update<T, MODE, ARITH, ISO, decltype(ftz)::value>(m0, m1, m2, a.k64, a.k32);
+                }
                 T nv;
                 if constexpr (MODE == MODE_REPLACE) {
                   nv = g;
-                  if (!CB::below(g, bnd)) {
+                  if (!(kGod64 ? d_below(g, bnd) : CB::below(g, bnd))) {
                     const int lz = L + i - lxy, gz = szd > 0 ? lz : BZ - 1 - lz;
                     nv = vmin<T, ARITH>(cap_value<T, ARITH>(capg + (long long)(z0 + gz) * a.plane +
                                                             (long long)(y0 + gyl) * a.px + (x0 + gxl)),
                                         g);
                   }
                 } else {
-                  nv = vmin<T, ARITH>(v, g);
+                  nv = kGod64 ? d_min(v, g) : vmin<T, ARITH>(v, g);
                 }
-                if (vdiffers<T, ARITH>(nv, v)) {
+                if (kGod64 ? d_differ(nv, v) : vdiffers<T, ARITH>(nv, v)) {
                   *p = nv;
                   cg |= bit;
                   T dv = T(0);
                   if (rec || change_may_exceed<T, ARITH>(v, nv, a.hmin, tmax)) {
                     dv = node_change<T, ARITH>(v, nv, a.hmin);
-                    tmax = vmax_nonneg<T, ARITH>(tmax, dv);
+                    tmax = kGod64 ? d_max(tmax, dv) : vmax_nonneg<T, ARITH>(tmax, dv);
                   }
                   if (rec) {
                     const int lz = L + i - lxy, q = (szd > 0 ? lz : BZ - 1 - lz) >> 3;

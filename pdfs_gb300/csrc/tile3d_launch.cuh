@@ -9,7 +9,7 @@ namespace pdfs {
 
 template <class T, int BX, int BY, int BZ, int MODE, int ARITH, bool ISO, bool OCT>
 static cudaError_t launch_t3(const SweepArgs &a, const Layout &L, int sms, cudaStream_t st, int *grid_used) {
-  using G = T3Geo<T, BX, BY, BZ>;
+  using G = T3GeoOf<T, BX, BY, BZ, ARITH>;
   auto kern = t3_sweep_kernel<T, BX, BY, BZ, MODE, ARITH, ISO, OCT>;
   CUtensorMap m;
   cudaError_t e = encode_field_map(&m, a.u, sizeof(T), L, a.nz + 2, G::W, G::RY, G::RZ);

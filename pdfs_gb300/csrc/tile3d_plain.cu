@@ -18,6 +18,10 @@ static int ordering_of(int sx, int sy, int sz) {
 template <int MODE>
 static cudaError_t plain64(int b, int bz, int arith, bool iso, const SweepArgs &a, const Layout &L, int sms,
                            cudaStream_t st, int *g) {
+  if (b == 8 && bz == 16) {
+    if (arith == ARITH_REF) return launch_t3<double, 8, 8, 16, MODE, ARITH_REF, false, true>(a, L, sms, st, g);
+    if (arith == ARITH_FAST) return launch_t3<double, 8, 8, 16, MODE, ARITH_FAST, false, true>(a, L, sms, st, g);
+  }
   if (b == 16 && bz == 32) {
     if (arith == ARITH_MIXED)
       return iso ? launch_t3<double, 16, 16, 32, MODE, ARITH_MIXED, true, true>(a, L, sms, st, g)
