@@ -100,6 +100,32 @@ __global__ void k_fill(T *p, size_t n, T v) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
+constexpr int kRowWarps = 8;  // rows of a CTA in the row kernels: one warp each
+
+// The padding of a row layout (everything outside the halo-padded grid) <- v, one
+// warp per row of the layout.  The grid itself is written by the load and by the
+// start of each phase, so filling it too only costs its bytes (768^3: 1.4 ms for
+// the three fields; the padding alone 0.2).
+template <class T>
+__global__ void __launch_bounds__(32 * kRowWarps) k_fill_pad(T *p, Layout L, int nx, int ny, int nz, T v) {
+  const long long r = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (r >= L.ry * (nz + 2)) return;
+  T *row = p + r * L.px;
+  const bool in = r % L.ry <= ny + 1;
+  const int lane = threadIdx.x & 31;
+  for (int q = lane; q < (in ? L.xo : 0); q += 32) row[q] = v;
+  for (long long q = (in ? L.xo + nx + 2 : 0) + lane; q < L.px; q += 32) row[q] = v;
+}
+
+template <class T>
+static void fill_padding(T *p, const Layout &L, const pdfs_grid &g, int sms, cudaStream_t st) {
+  if (L.zc)
+    k_fill<T><<<2 * sms, 256, 0, st>>>(p, L.elems, (T)INFINITY);
+  else
+    k_fill_pad<T><<<(unsigned)((L.ry * (g.nz + 2) + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, 0, st>>>(
+        p, L, g.nx, g.ny, g.nz, (T)INFINITY);
+}
+
 // reference layout (double) -> internal layout of T
 template <class T>
 __global__ void k_pack(const double *__restrict__ ref, T *__restrict__ dst, int nx, int ny, Layout L, int z0) {
@@ -108,19 +134,27 @@ __global__ void k_pack(const double *__restrict__ ref, T *__restrict__ dst, int 
   for (int x = threadIdx.x; x < nx + 2; x += blockDim.x) dst[L.index(x, y, z)] = (T)row[x];
 }
 
-// internal layout -> reference layout (double).  FP32 source: frozen nodes
-// (mask bit set) take the exact FP64 input instead of the rounded value.
+// internal layout -> reference layout (double), rows z0 (ny + 2) .. z1 (ny + 2),
+// one warp each.  FP32 source: frozen nodes (mask bit set) take the exact FP64
+// input instead of the rounded value.
 template <class T>
-__global__ void k_unpack(const T *__restrict__ src, Layout L, const double *__restrict__ in64, Layout L64,
-                         const uint32_t *__restrict__ fmask, MaskLayout M, double *__restrict__ ref, int nx, int ny,
-                         int z0) {
-  const int y = blockIdx.x, z = blockIdx.y + z0;
-  double *row = ref + ((size_t)z * (ny + 2) + y) * (size_t)(nx + 2);
-  for (int x = threadIdx.x; x < nx + 2; x += blockDim.x) {
-    double v = (double)src[L.index(x, y, z)];
+__global__ void __launch_bounds__(32 * kRowWarps) k_unpack(const T *__restrict__ src, Layout L,
+                                                           const double *__restrict__ in64, Layout L64,
+                                                           const uint32_t *__restrict__ fmask, MaskLayout M,
+                                                           double *__restrict__ ref, int nx, int ny, int z0, int z1) {
+  const long long r = (long long)z0 * (ny + 2) + (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (r >= (long long)z1 * (ny + 2)) return;
+  const int y = (int)(r % (ny + 2)), z = (int)(r / (ny + 2));
+  double *row = ref + r * (nx + 2);
+  const T *sp = src + L.index(0, y, z);
+  const long long dx = L.zc ? L.qz : 1;
+  const bool masked = fmask && y >= 1 && y <= ny;
+#pragma unroll 4
+  for (int x = threadIdx.x & 31; x < nx + 2; x += 32) {
+    double v = (double)sp[x * dx];
     if (L.zc) v = fabs(v);  // z-column fields mark frozen nodes with the sign
-    if (fmask && x >= 1 && x <= nx && y >= 1 && y <= ny) {
-      const uint32_t w = fmask[M.word(x, y, z)];
+    if (masked && x >= 1 && x <= nx) {
+      const uint32_t w = __ldg(fmask + M.word(x, y, z));
       if ((w >> ((x - 1) & 31)) & 1u) v = in64[L64.index(x, y, z)];
     }
     row[x] = v;
@@ -130,7 +164,6 @@ __global__ void k_unpack(const T *__restrict__ src, Layout L, const double *__re
 // internal layout of S -> internal layout of D, every halo-padded node
 // (one warp per halo-padded row: row r = blockIdx.x * 8 + warp is (y, z) =
 // (r % (ny + 2), r / (ny + 2)))
-constexpr int kRowWarps = 8;
 template <class S, class D>
 __global__ void __launch_bounds__(32 * kRowWarps) k_convert(const S *__restrict__ src, Layout Ls, D *__restrict__ dst,
                                                             Layout Ld, int nx, int ny, int nz) {
@@ -238,76 +271,123 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_widen_pair(const float *__re
   }
 }
 
+// float -> double by its bits, off the FP64 pipe (no conversion left even as a
+// fallback: the compiler would run it beside the fast form and select)
+__device__ __forceinline__ double widen_bits(float f) {
+  const float g = f * 0x1p64f;  // a subnormal's exponent, exact
+  const bool sub = (__float_as_uint(f) & 0x7f800000u) == 0u;
+  const unsigned b = __float_as_uint(sub ? g : f), m = b & 0x7fffffffu;
+  unsigned bias = 0x38000000u;
+  if (sub) bias -= 64u << 20;
+  if (m == 0u) bias = 0u;
+  if (m >= 0x7f800000u) bias = 0x70000000u;  // infinity, NaN: exponent 255 -> 2047
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + bias)), (int)(m << 29));
+}
+
 // pair working field -> reference layout: hi + lo (exact in FP64) for the
-// updated nodes; frozen nodes and the halo take the exact FP64 input
-__global__ void k_unpack_pair(const double *__restrict__ src, Layout L, const double *__restrict__ in64,
-                              const uint32_t *__restrict__ fmask, MaskLayout M, double *__restrict__ ref, int nx,
-                              int ny, int nz, int z0) {
-  const int y = blockIdx.x, z = blockIdx.y + z0;
-  double *row = ref + ((size_t)z * (ny + 2) + y) * (size_t)(nx + 2);
-  for (int x = threadIdx.x; x < nx + 2; x += blockDim.x) {
-    const long long i = L.index(x, y, z);
-    const bool interior = x >= 1 && x <= nx && y >= 1 && y <= ny && z >= 1 && z <= nz;
-    bool frz = !interior;
-    if (interior && fmask) {
-      const uint32_t w = fmask[M.word(x, y, z)];
-      frz = (w >> ((x - 1) & 31)) & 1u;
+// updated nodes; frozen nodes and the halo take the exact FP64 input.  Rows
+// z0 (ny + 2) .. z1 (ny + 2), one warp each, four loads in flight before the first
+// is used.  Two conversions and an addition are three FP64-pipe operations a node,
+// which is what bounds a plain copy loop here (2.5 ms at 768^3 however the loads are
+// laid out): widening by the bits leaves the addition (1.7 ms).
+__global__ void __launch_bounds__(32 * kRowWarps) k_unpack_pair(const double *__restrict__ src, Layout L,
+                                                                const double *__restrict__ in64,
+                                                                const uint32_t *__restrict__ fmask, MaskLayout M,
+                                                                double *__restrict__ ref, int nx, int ny, int nz,
+                                                                int z0, int z1) {
+  const long long r = (long long)z0 * (ny + 2) + (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (r >= (long long)z1 * (ny + 2)) return;
+  const int y = (int)(r % (ny + 2)), z = (int)(r / (ny + 2));
+  double *row = ref + r * (nx + 2);
+  const long long i0 = L.index(0, y, z), dx = L.zc ? L.qz : 1;
+  const bool irow = y >= 1 && y <= ny && z >= 1 && z <= nz;
+  for (int xb = threadIdx.x & 31; xb < nx + 2; xb += 128) {
+    double v[4];
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int x = xb + 32 * k;
+      w[k] = 1u;
+      if (x < nx + 2) {
+        v[k] = src[i0 + x * dx];
+        if (irow && x >= 1 && x <= nx) w[k] = fmask ? __ldg(fmask + M.word(x, y, z)) >> ((x - 1) & 31) : 0u;
+      }
     }
-    const double v = src[i];
-    row[x] = frz ? in64[i] : (double)p_hi(v) + (double)p_lo(v);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int x = xb + 32 * k;
+      if (x < nx + 2) row[x] = (w[k] & 1u) ? in64[i0 + x * dx] : widen_bits(p_hi(v[k])) + widen_bits(p_lo(v[k]));
+    }
   }
 }
 
 // Per 8^3 block: the smallest input value (the replace-update's cap) of the
 // nodes the sweeps update (+inf if every node is frozen), and the same rounded
-// down to float.  One warp per block, blocks b0 .. b1-1: lane (x, y) = (lane %
-// 8, lane / 8) of a 8 x 4 quarter plane loads its 16 nodes before reducing.
-__global__ void k_block_capmin(const double *__restrict__ in64, Layout L, const uint32_t *__restrict__ fmask,
-                               MaskLayout M, int nx, int ny, int nz, int nbx, int nby, long long b0, long long b1,
-                               double *__restrict__ b64, float *__restrict__ b32) {
-  const int lane = threadIdx.x & 31;
-  for (long long b = b0 + ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5); b < b1;
-       b += ((long long)gridDim.x * blockDim.x) >> 5) {
-    const int bx = (int)(b % nbx), by = (int)((b / nbx) % nby), bz = (int)(b / ((long long)nbx * nby));
-    const int x = 1 + bx * 8 + (lane & 7);
-    double v[16];
-    bool use[16];
+// down to float.  One CTA per four blocks along x, block layers bz0 and up; warp =
+// plane, lane = x, so that a load is 32 nodes of one row, its frozen bits are one
+// word, and a CTA's 64 rows are in flight together (a warp per block, 8 nodes of 4
+// rows a load: 1.65 ms at 768^3; a warp per four blocks: 1.10, and 20 us against 9
+// on grids to 160^3; this 0.84).
+__global__ void __launch_bounds__(256) k_block_capmin(const double *__restrict__ in64, Layout L,
+                                                      const uint32_t *__restrict__ fmask, MaskLayout M, int nx, int ny,
+                                                      int nz, int nbx, int nby, int bz0, double *__restrict__ b64,
+                                                      float *__restrict__ b32) {
+  __shared__ double s_m[8][4];
+  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5, nwx = (nbx + 3) / 4;
+  const int wx = (int)(blockIdx.x % nwx), by = (int)((blockIdx.x / nwx) % nby);
+  const int bz = bz0 + (int)(blockIdx.x / ((unsigned)nwx * (unsigned)nby));
+  const int x = 1 + wx * 32 + lane, y0 = 1 + by * 8, z = 1 + bz * 8 + k;
+  double m = INFINITY;
+  if (z <= nz) {
+    const long long dy = L.index(0, 1, 0) - L.index(0, 0, 0);
+    const double *p = in64 + L.index(x, y0, z);
+    const uint32_t *f = fmask ? fmask + M.word(1 + wx * 32, y0, z) : nullptr;
+    double v[8];
+    uint32_t w[8];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int y = 1 + by * 8 + (lane >> 3) + 4 * (k & 1), z = 1 + bz * 8 + (k >> 1);
-      use[k] = x <= nx && y <= ny && z <= nz;
-      v[k] = use[k] ? in64[L.index(x, y, z)] : INFINITY;
-      if (use[k] && fmask) use[k] = !((fmask[M.word(x, y, z)] >> ((x - 1) & 31)) & 1u);
+    for (int j = 0; j < 8; ++j) {
+      v[j] = x <= nx && y0 + j <= ny ? p[j * dy] : INFINITY;
+      w[j] = f && y0 + j <= ny ? __ldg(f + j) : 0u;
     }
-    double m = INFINITY;
 #pragma unroll
-    for (int k = 0; k < 16; ++k)
-      if (use[k] && dkey(v[k]) < dkey(m)) m = v[k];  // integer keys: off the FP64 pipe
+    for (int j = 0; j < 8; ++j)
+      if (!((w[j] >> lane) & 1u) && dkey(v[j]) < dkey(m)) m = v[j];  // integer keys: off the FP64 pipe
+  }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double o = __shfl_xor_sync(0xffffffffu, m, off);
-      m = dkey(o) < dkey(m) ? o : m;
-    }
-    if (lane == 0) {
-      b64[b] = m;
-      b32[b] = __double2float_rd(m);
-    }
+  for (int off = 4; off > 0; off >>= 1) {
+    const double o = __shfl_xor_sync(0xffffffffu, m, off);
+    m = dkey(o) < dkey(m) ? o : m;
+  }
+  if ((lane & 7) == 0) s_m[k][lane >> 3] = m;
+  __syncthreads();
+  const int bx = wx * 4 + (int)threadIdx.x;
+  if (threadIdx.x < 4 && bx < nbx) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (dkey(s_m[j][threadIdx.x]) < dkey(m)) m = s_m[j][threadIdx.x];
+    const long long b = ((long long)bz * nby + by) * nbx + bx;
+    b64[b] = m;
+    b32[b] = __double2float_rd(m);
   }
 }
 
-// uint8 mask in the reference layout -> frozen bitmask (interior nodes only)
-__global__ void k_pack_mask(const uint8_t *__restrict__ m, uint32_t *__restrict__ bits, MaskLayout M, int nx,
-                            int ny) {
-  const int y = blockIdx.x + 1, z = blockIdx.y + 1;  // interior rows only
+// uint8 mask in the reference layout -> frozen bitmask (interior nodes only):
+// one warp per row, a byte a lane and a ballot per word
+__global__ void __launch_bounds__(32 * kRowWarps) k_pack_mask(const uint8_t *__restrict__ m,
+                                                              uint32_t *__restrict__ bits, MaskLayout M, int nx,
+                                                              int ny, int nz) {
+  const long long r = (long long)blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (r >= (long long)ny * nz) return;
+  const int y = 1 + (int)(r % ny), z = 1 + (int)(r / ny);  // interior rows only
+  const int lane = threadIdx.x & 31;
   const uint8_t *row = m + ((size_t)z * (ny + 2) + y) * (size_t)(nx + 2);
+  uint32_t *out = bits + M.word(1, y, z);
   const int nwords = (nx + 31) / 32;
-  for (int w = threadIdx.x; w < nwords; w += blockDim.x) {
-    uint32_t v = 0;
-    for (int b = 0; b < 32; ++b) {
-      const int x = 1 + w * 32 + b;
-      if (x <= nx && row[x]) v |= 1u << b;
-    }
-    bits[M.word(1 + w * 32, y, z)] = v;
+#pragma unroll 4
+  for (int w = 0; w < nwords; ++w) {
+    const int x = 1 + w * 32 + lane;
+    const uint32_t v = __ballot_sync(0xffffffffu, x <= nx && row[x]);
+    if (lane == 0) out[(long long)w * M.fy] = v;
   }
 }
 
@@ -845,9 +925,9 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
     return fail(e);
   const auto t_alloc = std::chrono::steady_clock::now();
   // padding outside the halo-padded grid is never written by the sweeps; fill it with +inf once
-  if (c->in64) k_fill<double><<<2 * c->sms, 256, 0, c->st>>>(c->in64, c->L64.elems, INFINITY);
-  if (c->u64) k_fill<double><<<2 * c->sms, 256, 0, c->st>>>(c->u64, c->L64.elems, INFINITY);
-  if (c->u32) k_fill<float><<<2 * c->sms, 256, 0, c->st>>>(c->u32, c->L32.elems, INFINITY);
+  if (c->in64) fill_padding(c->in64, c->L64, c->g, c->sms, c->st);
+  if (c->u64) fill_padding(c->u64, c->L64, c->g, c->sms, c->st);
+  if (c->u32) fill_padding(c->u32, c->L32, c->g, c->sms, c->st);
   if ((e = cudaMemsetAsync(c->fmask, 0, c->M.words * 4, c->st)) != cudaSuccess) return fail(e);
   if ((e = cudaEventCreate(&c->e0)) != cudaSuccess) return fail(e);
   if ((e = cudaEventCreate(&c->e1)) != cudaSuccess) return fail(e);
@@ -975,11 +1055,10 @@ static int load_impl(pdfs_ctx *c, const double *field, const uint8_t *frozen, do
       CK(cudaMemcpyAsync((void *)m, frozen, n, cudaMemcpyHostToDevice, c->st));
       CK(handoff(c->slab_ev[pdfs_ctx::kSlabs]));
     }
-    dim3 mg(g.ny, g.nz);
-    k_pack_mask<<<mg, 64, 0, ks>>>(m, c->fmask, c->M, g.nx, g.ny);
+    k_pack_mask<<<(unsigned)(((long long)g.ny * g.nz + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, 0, ks>>>(
+        m, c->fmask, c->M, g.nx, g.ny, g.nz);
     CK(cudaGetLastError());
   }
-  const long long blocks_per_z = (long long)c->nbx * c->nby;
   int bz_done = 0;
   for (int z0 = 0, k = 0; z0 < planes; z0 += per, ++k) {
     const int z1 = std::min(planes, z0 + per);
@@ -995,9 +1074,9 @@ static int load_impl(pdfs_ctx *c, const double *field, const uint8_t *frozen, do
       // block bz holds planes 8 bz + 1 .. min(8 bz + 8, nz): complete once plane z1 - 1 is packed
       const int bz_ready = z1 >= g.nz + 1 ? c->nbz : std::min(c->nbz, (z1 - 1) / 8);
       if (bz_ready > bz_done) {
-        k_block_capmin<<<8 * c->sms, 256, 0, ks>>>(c->in64, c->L64, use_mask ? c->fmask : nullptr, c->M, g.nx,
-                                                        g.ny, g.nz, c->nbx, c->nby, bz_done * blocks_per_z,
-                                                        bz_ready * blocks_per_z, c->bcap64, c->bcap32);
+        const long long ctas = (long long)((c->nbx + 3) / 4) * c->nby * (bz_ready - bz_done);
+        k_block_capmin<<<(unsigned)ctas, 256, 0, ks>>>(c->in64, c->L64, use_mask ? c->fmask : nullptr, c->M, g.nx, g.ny,
+                                                       g.nz, c->nbx, c->nby, bz_done, c->bcap64, c->bcap32);
         CK(cudaGetLastError());
         bz_done = bz_ready;
       }
@@ -1542,13 +1621,14 @@ static int store_impl(pdfs_ctx *c, double *field, double *ms_d2h) {
   const uint32_t *fm = c->has_mask ? c->fmask : nullptr;
   for (int z0 = 0, k = 0; z0 < planes; z0 += per, ++k) {
     const int z1 = std::min(planes, z0 + per);
-    dim3 grid(g.ny + 2, z1 - z0);
+    const unsigned grid = (unsigned)(((long long)(g.ny + 2) * (z1 - z0) + kRowWarps - 1) / kRowWarps);
+    constexpr int kT = 32 * kRowWarps;
     if (c->last_prec == 1 && c->o.arith == PDFS_ARITH_PAIR)
-      k_unpack_pair<<<grid, 128, 0, c->st>>>(c->u64, c->L64, c->in64, fm, c->M, dst, g.nx, g.ny, g.nz, z0);
+      k_unpack_pair<<<grid, kT, 0, c->st>>>(c->u64, c->L64, c->in64, fm, c->M, dst, g.nx, g.ny, g.nz, z0, z1);
     else if (c->last_prec == 1)
-      k_unpack<double><<<grid, 128, 0, c->st>>>(c->u64, c->L64, c->in64, c->L64, nullptr, c->M, dst, g.nx, g.ny, z0);
+      k_unpack<double><<<grid, kT, 0, c->st>>>(c->u64, c->L64, c->in64, c->L64, nullptr, c->M, dst, g.nx, g.ny, z0, z1);
     else
-      k_unpack<float><<<grid, 128, 0, c->st>>>(c->u32, c->L32, c->in64, c->L64, fm, c->M, dst, g.nx, g.ny, z0);
+      k_unpack<float><<<grid, kT, 0, c->st>>>(c->u32, c->L32, c->in64, c->L64, fm, c->M, dst, g.nx, g.ny, z0, z1);
     CK(cudaGetLastError());
     if (!dev) {
       if (pipe) {
