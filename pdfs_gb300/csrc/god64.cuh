@@ -12,9 +12,13 @@
 // System/6000 processor", IBM J. Res. Dev. 34, 1990: with y = RN(1/b), q within
 // an ulp of a/b and r = a - b q exact, RN(q + r y) = RN(a/b)), and a square root
 // starts from an FP32 reciprocal root refined to 45 bits in FP32: 61 and 25
-// FP64 operations an update.  Rounding by rounding, god64_ref is god_ref64.
-// One warp, a three-term update: 4585 cycles against 6631 (reference), 2043
-// against 3950 (fast).
+// FP64 operations an update.  A node with three terms is mostly known to have them
+// before its two-term solution is: 44 and 16.  Rounding by rounding, god64_ref is
+// god_ref64.
+// One warp, a three-term update: 3583 cycles against 6631 (reference), 1480 against
+// 3950 (fast); 4585 and 2043 with the two-term solution always first (a 384^3
+// sweep, 8 x 8 x 16 bricks: 10.1 -> 8.8 ms reference, 4.56 -> 4.04 fast; 64^3, where a
+// level's lanes rarely agree, even).
 //
 // They take finite or +inf non-negative values; anything else (negative
 // values, NaN) goes to the plain solvers.
@@ -114,17 +118,46 @@ __device__ __forceinline__ int sort64(double &m0, double &m1, double &m2) {
   return 2 * a0 + (a1 > a2 ? 1 : 0);  // a0, then whether the other two are swapped
 }
 
+// v >= 0 as a float, cut off (0 below the normal floats, +inf above)
+__device__ __forceinline__ float d_float(double v) {
+  const unsigned h = d_hi(v);
+  const float f = __uint_as_float(((h - 0x38000000u) << 3) | (d_lo(v) >> 29));
+  return h < 0x38100000u ? 0.0f : h >= 0x47f00000u ? INFINITY : f;
+}
+
+// Does the two-term solution of god_ref64 surely exceed m2, whatever its rounding?
+// It does in exact arithmetic where T = w0 (m2 - m0)^2 + w1 (m2 - m1)^2 < 1, and by
+// at least (1 - T) / (2 sqrt(w0 + w1)).  With M = m1 + d0 + d1, dm = min(d0, d1) and
+// R = M / dm, its rounding error is below 16 u M^2 / dm, u = 2^-53 (the
+// discriminant's terms are products of the minima, 8 u M^2 in all, and its root is
+// at least d1), so 1 - T > 1e-14 R^2 is enough; T itself, from the minima cut to
+// floats, is good to 4 times 2^-22 R and some 2^-20.  1e-5 + 2e-6 R covers both (it
+// is below 1, so that anything is sure at all, only for R < 5e5).  True spares the
+// two-term solution: 17 FP64 operations of 61.
+__device__ __forceinline__ bool three_terms(double m0, double m1, double m2, const GodPerm64 &k) {
+  const float f0 = d_float(m0), f1 = d_float(m1), f2 = d_float(m2);
+  const float b = __fmul_rn(__fsub_rn(f2, f0), k.r0), c = __fmul_rn(__fsub_rn(f2, f1), k.r1);
+  const float T = __fmaf_rn(b, b, __fmul_rn(c, c));
+  return T < 1.0f - __fmaf_rn(__fmaf_rn(f1, k.rm, k.rd), 2e-6f, 1e-5f);  // (false for infinities and NaN)
+}
+
 // god_ref64 on sorted minima: the same roundings.  A doubled product is a
 // multiply-add with 2 (exact), -x - x is -2 x.
 __device__ __forceinline__ double god64_ref(double m0, double m1, double m2, const GodPerm64 &k, bool &ok) {
   double u = __dadd_rn(m0, k.d0);
   if (d_less(m1, u)) {
     const double m00 = __dmul_rn(m0, m0), m11 = __dmul_rn(m1, m1), p01 = __dmul_rn(m0, m1);
-    double t = __fma_rn(2.0, p01, -m00);
-    t = __dadd_rn(__dadd_rn(__dsub_rn(t, m11), k.q0), k.q1);
     const double m1q0 = __dmul_rn(m1, k.q0), m0q1 = __dmul_rn(m0, k.q1);
-    u = div64(__dadd_rn(__dadd_rn(m1q0, m0q1), __dmul_rn(k.d01, sqrt64<true>(t, ok))), k.s, k.is, ok);
-    if (d_less(m2, u)) {
+    const unsigned lanes = __activemask();
+    bool three = d_less(m2, u) && three_terms(m0, m1, m2, k);
+    if (!three) {
+      double t = __fma_rn(2.0, p01, -m00);
+      t = __dadd_rn(__dadd_rn(__dsub_rn(t, m11), k.q0), k.q1);
+      u = div64(__dadd_rn(__dadd_rn(m1q0, m0q1), __dmul_rn(k.d01, sqrt64<true>(t, ok))), k.s, k.is, ok);
+      three = d_less(m2, u);
+    }
+    __syncwarp(lanes);  // one pass over the third term for all (see god64_node)
+    if (three) {
       const double m22 = __dmul_rn(m2, m2), p02 = __dmul_rn(m0, m2), p12 = __dmul_rn(m1, m2);
       double r = __dsub_rn(__dmul_rn(-m00, k.q1), __dmul_rn(m00, k.q2));
       r = __fma_rn(2.0, __dmul_rn(p01, k.q2), r);
@@ -144,18 +177,29 @@ __device__ __forceinline__ double god64_ref(double m0, double m1, double m2, con
   return u;
 }
 
-// god_fast64 on sorted minima, with reciprocals for its divisions.
+// god_fast64 on sorted minima, with reciprocals for its divisions and the
+// three-term solution first: the two-term one exceeds m2 exactly where the
+// three-term one does (to rounding, and where they meet they are equal), so a node
+// with three terms needs no other.
 __device__ __forceinline__ double god64_fast(double m0, double m1, double m2, const GodPerm64 &k, bool &ok) {
   double u = __dadd_rn(m0, k.d0);
   if (d_less(m1, u)) {
     const double a = __dsub_rn(m1, m0), aa = __dmul_rn(a, a);
-    u = __fma_rn(__fma_rn(a, k.w1, sqrt64<false>(__fma_rn(-aa, k.w01, k.ws), ok)), k.iws, m0);
+    const unsigned lanes = __activemask();
+    bool two = true;
     if (d_less(m2, u)) {
       const double b = __dsub_rn(m2, m0);
       const double B = __fma_rn(a, k.w1, __dmul_rn(b, k.w2));
       const double C = __fma_rn(aa, k.w1, __fma_rn(__dmul_rn(b, b), k.w2, -1.0));
-      u = __fma_rn(__dadd_rn(B, sqrt64<false>(__fma_rn(B, B, __dmul_rn(-k.wsum, C)), ok)), k.iwsum, m0);
+      const double D = __fma_rn(B, B, __dmul_rn(-k.wsum, C));
+      if (__double_as_longlong(D) > 0) {
+        const double v = __fma_rn(__dadd_rn(B, sqrt64<false>(D, ok)), k.iwsum, m0);
+        two = !d_less(m2, v);
+        if (!two) u = v;
+      }
     }
+    __syncwarp(lanes);
+    if (two) u = __fma_rn(__fma_rn(a, k.w1, sqrt64<false>(__fma_rn(-aa, k.w01, k.ws), ok)), k.iws, m0);
   }
   return u;
 }

@@ -42,7 +42,8 @@ struct GodPerm64 {
   double w1, w2, w01;    // w0 w1
   double ws, iws;        // w0 + w1, 1 / ws
   double wsum, iwsum;    // w of all axes, 1 / wsum
-  double pad;            // rows of 21 doubles: six of them read at once share no bank
+  float r0, r1, rm, rd;  // 1 / d0, 1 / d1, 1 / min(d0, d1), (d0 + d1) / min(d0, d1)
+  double pad;            // rows of 23 doubles: six of them read at once share no bank
 };
 
 // Per-sweep constants of the local solver.

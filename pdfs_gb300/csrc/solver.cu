@@ -502,6 +502,10 @@ static void fill_perm(const pdfs_grid &g, GodPerm64 out[6]) {
       p.iws = 1.0 / p.ws;
       p.wsum = wsum;
       p.iwsum = 1.0 / wsum;
+      p.r0 = (float)(1.0 / d0);
+      p.r1 = (float)(1.0 / d1);
+      p.rm = (float)(1.0 / std::min(d0, d1));
+      p.rd = (float)((d0 + d1) / std::min(d0, d1));
     }
 }
 
@@ -671,11 +675,11 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 //     leaves room for two CTAs, and a brick reads its halo (27 % more bytes): what
 //     bricks save in the chain they lose once the chip is full.
 //   reference and fast: bricks of 8 x 8 x 16 with the solvers of god64.cuh.
-//     Reference 0.54 / 3.7 / 10.1 / 3.6 / -, pencils 1.35 / 10.5 / 18.7 / - / -; fast
-//     0.29 / 1.7 / 4.6 / 1.8 / -, pencils 0.82 / 5.6 / 10.4 / - / -.  A level costs one
-//     warp some 60 (25) FP64 operations of 64 cycles each however few of its lanes
-//     hold a node, so small faces, which lag their upwind bricks by fewer levels, win:
-//     16 x 16 x 16 bricks take 0.73 / 4.5 / 10.6 and 0.36 / 2.0 / 5.0.
+//     Reference 0.54 / 3.3 / 8.8 / 3.5 / -, pencils 1.35 / 10.5 / 18.7 / - / -; fast
+//     0.29 / 1.5 / 4.0 / 1.8 / -, pencils 0.82 / 5.6 / 10.4 / - / -.  A level costs one
+//     warp 16 to 61 FP64 operations of 64 cycles each however few of its lanes hold
+//     a node, so small faces, which lag their upwind bricks by fewer levels, win:
+//     16 x 16 x 16 bricks take 5 to 50 % more.
 constexpr long long kPairBrickNodes = 1ll << 26;
 
 static void pick_tiles(pdfs_ctx *c) {
