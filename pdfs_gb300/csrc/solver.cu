@@ -666,8 +666,13 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 //
 // Plain sweeps of the pencil tiles (no mask, no block changes), ms a sweep on
 // 64^3 / 251 x 233 x 241 / 384^3 / 1000 x 60 x 50 / 768^3 nodes:
-//   FP32: bricks of 16 x 16 x 32, 0.079 / 0.37 / 0.68 / 0.51 / 3.15, against 0.120 /
-//     0.52 / 1.04 / 0.71 / 3.94 on pencils.
+//   FP32: bricks of 8 x 8 x 32 while a level of the sweep holds at most 30000 nodes on
+//     average, 0.074 / 0.34 / (0.75) / 0.47 / (4.1), else of 16 x 16 x 32, (0.079) /
+//     (0.37) / 0.68 / (0.51) / 3.15; pencils take 0.120 / 0.52 / 1.04 / 0.71 / 3.94.
+//     Small faces shorten the chain (8 levels a brick crossed instead of 16), but
+//     their halos are read and their faces mailed twice as often, which is what counts
+//     once the levels fill the chip: both are even at 288^3 (27600 nodes a level: 0.444
+//     and 0.451), 322^3 (34600) takes 0.57 and 0.54, 512 x 512 x 128 (29100) 0.64 and 0.73.
 //   pairs and mixed: bricks of 16 x 16 x 32 up to 2^26 nodes, pencils above.  Pairs
 //     0.117 / 0.53 / 1.11 / 0.75 / 7.3, pencils 0.164 / 0.70 / 1.25 / 0.96 / 5.6; mixed
 //     0.175 / 0.83 / 1.71 / - / 9.8 and 0.214 / 1.00 / 1.79 / - / 8.5; both are even at
@@ -681,6 +686,7 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 //     a node, so small faces, which lag their upwind bricks by fewer levels, win:
 //     16 x 16 x 16 bricks take 5 to 50 % more.
 constexpr long long kPairBrickNodes = 1ll << 26;
+constexpr long long kSmallBrickLevel = 30000;
 
 static void pick_tiles(pdfs_ctx *c) {
   const int t32 = c->o.tile & 0xff, t64 = (c->o.tile >> 8) & 0xff;
@@ -693,11 +699,17 @@ static void pick_tiles(pdfs_ctx *c) {
     p.nt[1] = (c->g.ny + b - 1) / b;
     p.nt[2] = (c->g.nz + bz - 1) / bz;
   };
-  if (tile32(c->t32).pencil) set(c->plain32, 16, 32);
+  const long long nodes = (long long)c->g.nx * c->g.ny * c->g.nz;
+  if (tile32(c->t32).pencil) {
+    if (nodes <= kSmallBrickLevel * ((long long)c->g.nx + c->g.ny + c->g.nz))
+      set(c->plain32, 8, 32);
+    else
+      set(c->plain32, 16, 32);
+  }
   if (tile64(c->t64).pencil) {
     if (c->o.arith == PDFS_ARITH_REFERENCE || c->o.arith == PDFS_ARITH_FAST)
       set(c->plain64, 8, 16);
-    else if ((long long)c->g.nx * c->g.ny * c->g.nz <= kPairBrickNodes)
+    else if (nodes <= kPairBrickNodes)
       set(c->plain64, 16, 32);
   }
 }

@@ -45,6 +45,9 @@ cudaError_t launch_sweep_plain(int which, int b, int bz, int arith, bool iso, co
   a.tflag = nullptr;  // no later sweep waits for its flags
   a.nticket = nullptr;
   a.tact = nullptr;
+  if (which == 0 && b == 8 && bz == 32)
+    return iso ? launch_t3<float, 8, 8, 32, MODE_MIN, ARITH_FAST, true, true>(a, L, sms, st, g)
+               : launch_t3<float, 8, 8, 32, MODE_MIN, ARITH_FAST, false, true>(a, L, sms, st, g);
   if (which == 0 && b == 16 && bz == 32)
     return iso ? launch_t3<float, 16, 16, 32, MODE_MIN, ARITH_FAST, true, true>(a, L, sms, st, g)
                : launch_t3<float, 16, 16, 32, MODE_MIN, ARITH_FAST, false, true>(a, L, sms, st, g);

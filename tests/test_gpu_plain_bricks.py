@@ -13,7 +13,8 @@ from pdfs_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(1, 1, 1), (16, 16, 32), (17, 16, 33), (15, 31, 31), (16, 1, 65), (33, 50, 8), (50, 43, 52), (97, 33, 64)]
+SHAPES = [(1, 1, 1), (8, 8, 32), (9, 8, 33), (7, 15, 31), (16, 16, 32), (17, 16, 33), (15, 31, 31), (16, 1, 65),
+          (33, 50, 8), (50, 43, 52), (97, 33, 64)]
 SPACINGS = [(1.0, 1.0, 1.0), (0.7, 1.0, 0.5)]
 
 
@@ -40,6 +41,13 @@ def test_fp32_sweeps_equal_column_sweeps(shape, sp):
         a, b = (sweeps(w, sp, frozen, precision=L.PREC_FP32, tile=t) for t in (10, 4))
         assert a[0] == b[0]
         assert a[1] == pytest.approx(b[1], rel=1e-6)  # the change of a node, in either kernel's rounding
+
+
+def test_fp32_sweeps_of_wide_levels():
+    """A grid past the level width of the small bricks (37000 nodes a level)."""
+    w = field((347, 323, 329), (1.0, 1.0, 1.0))
+    a, b = (sweeps(w, (1.0, 1.0, 1.0), w.frozen, precision=L.PREC_FP32, tile=t) for t in (10, 4))
+    assert a[0] == b[0]
 
 
 @pytest.mark.parametrize("arith", [L.ARITH_PAIR, L.ARITH_MIXED])
