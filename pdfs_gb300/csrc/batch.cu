@@ -25,7 +25,10 @@ namespace {
 struct BatchState {
   int n = 0;
   int dev = 0, sms = 0;
-  cudaStream_t st = nullptr;
+  Handles hd;
+  cudaStream_t st = nullptr;  // hd.st
+  void *block = nullptr;      // the d_ arrays but d_prog
+  size_t block_bytes = 0;
   SweepArgs *d_args = nullptr;
   CUtensorMap *d_maps = nullptr;
   int2 *d_tickets = nullptr;
@@ -44,19 +47,11 @@ struct BatchState {
   ~BatchState() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
-    cudaFree(d_args);
-    cudaFree(d_maps);
-    cudaFree(d_tickets);
-    cudaFree(d_desc);
+    if (st) cudaStreamSynchronize(st);
     cudaFree(d_prog);
-    cudaFree(d_chg);
-    cudaFree(d_err);
-    cudaFree(d_ticket);
-    cudaFree(d_done);
-    cudaFree(d_round);
-    if (h_chg) cudaFreeHost(h_chg);
-    if (h_err) cudaFreeHost(h_err);
-    if (st) cudaStreamDestroy(st);
+    block_give(dev, block, block_bytes);
+    if (h_err && (char *)h_err != hd.pinned) cudaFreeHost(h_err);
+    handles_give(dev, &hd);
   }
 };
 
@@ -472,21 +467,39 @@ extern "C" int pdfs_solve_batch(int n, const pdfs_grid *grids, double *const *fi
       return cleanup(cuda_status(e));   \
     }                                   \
   } while (0)
-  BQ(cudaStreamCreateWithFlags(&B.st, cudaStreamNonBlocking));
+  BQ(handles_take(B.dev, &B.hd));
+  B.st = B.hd.st;
   size_t total_cols = 0;  // tickets: columns of a sweep, or pencils of a round's 8 sweeps
   for (auto *c : ctx) total_cols += 8 * std::max((size_t)c->L32.ncx * c->L32.ncy, (size_t)c->L64.ncx * c->L64.ncy);
-  BQ(cudaMalloc(&B.d_args, sizeof(SweepArgs) * n));
-  BQ(cudaMalloc(&B.d_maps, sizeof(CUtensorMap) * 3 * n));
-  BQ(cudaMalloc(&B.d_tickets, sizeof(int2) * total_cols));
-  BQ(cudaMalloc(&B.d_desc, sizeof(BatchDesc)));
-  BQ(cudaMalloc(&B.d_chg, sizeof(unsigned long long) * 8 * n));
-  BQ(cudaMalloc(&B.d_err, 16));
-  BQ(cudaMalloc(&B.d_ticket, 16));
-  BQ(cudaMalloc(&B.d_done, sizeof(int) * 8 * n));
-  BQ(cudaMalloc(&B.d_round, 16));
-  BQ(cudaMemset(B.d_err, 0, 16));
-  BQ(cudaHostAlloc(&B.h_chg, sizeof(unsigned long long) * 8 * n, cudaHostAllocDefault));
-  BQ(cudaHostAlloc(&B.h_err, 16, cudaHostAllocDefault));
+  {
+    std::vector<std::pair<void **, size_t>> plan;
+    auto want = [&](auto **p, size_t bytes) { plan.emplace_back((void **)p, (bytes + 255) & ~(size_t)255); };
+    want(&B.d_args, sizeof(SweepArgs) * n);
+    want(&B.d_maps, sizeof(CUtensorMap) * 3 * n);
+    want(&B.d_tickets, sizeof(int2) * total_cols);
+    want(&B.d_desc, sizeof(BatchDesc));
+    want(&B.d_chg, sizeof(unsigned long long) * 8 * n);
+    want(&B.d_err, 16);
+    want(&B.d_ticket, 16);
+    want(&B.d_done, sizeof(int) * 8 * n);
+    want(&B.d_round, 16);
+    for (auto &r : plan) B.block_bytes += r.second;
+    BQ(block_take(B.dev, &B.block, B.block_bytes));
+    char *p = (char *)B.block;
+    for (auto &r : plan) {
+      *r.first = p;
+      p += r.second;
+    }
+  }
+  BQ(cudaMemsetAsync(B.d_err, 0, 16, B.st));
+  BQ(cudaStreamSynchronize(B.st));
+  {
+    const size_t host = 64 + sizeof(unsigned long long) * 8 * n;
+    void *p = B.hd.pinned;
+    if (host > kPinned) BQ(cudaHostAlloc(&p, host, cudaHostAllocDefault));
+    B.h_err = (int *)p;
+    B.h_chg = (unsigned long long *)((char *)p + 64);
+  }
   double kms32 = 0, kms64 = 0;
   int launches = 0;
   std::vector<int> all(n);

@@ -191,12 +191,37 @@ inline int mailbox_chunks(int nz) { return (nz + 32 + kMailboxChunk - 1) / kMail
 
 }  // namespace pdfs
 
+namespace pdfs {
+
+// The CUDA objects a solve needs beside device memory.  Making and destroying a
+// set costs some 0.1 ms (the pinned block most of it), so idle sets are pooled
+// (solver.cu): a taken set belongs to its taker alone until it is given back,
+// with its streams idle.
+constexpr int kSlabs = 32;
+constexpr size_t kPinned = 16384;
+struct Handles {
+  cudaStream_t st = nullptr;
+  cudaEvent_t ev[8] = {};
+  char *pinned = nullptr;  // kPinned bytes
+  // load / store pipeline, made on first use
+  cudaStream_t st2 = nullptr;
+  cudaEvent_t slab_ev[kSlabs + 1] = {};
+};
+cudaError_t handles_take(int dev, Handles *h);
+// Device memory from the cache of idle blocks, or new; given back idle.
+cudaError_t block_take(int dev, void **out, size_t bytes);
+void block_give(int dev, void *p, size_t bytes);
+void handles_give(int dev, Handles *h);  // waits for its streams; destroyed instead if they hold an error
+
+}  // namespace pdfs
+
 // The context behind the opaque pdfs_ctx handle of the C ABI.
 struct pdfs_ctx {
   pdfs_grid g{};
   pdfs_opts o{};
   int dev = 0, sms = 0;
-  cudaStream_t st = nullptr;
+  pdfs::Handles hd;
+  cudaStream_t st = nullptr;  // hd.st
   int t32 = 1, t64 = 1;
   pdfs::Layout L32, L64;
   pdfs::MaskLayout M;
@@ -232,7 +257,7 @@ struct pdfs_ctx {
   size_t mailbox_bytes = 0;
   size_t progress_ints = 0;
   pdfs::DevStatus *dstat = nullptr;
-  pdfs::DevStatus *hstat = nullptr;  // pinned
+  pdfs::DevStatus *hstat = nullptr;  // hd.pinned
   // 8^3 block bookkeeping for the scheduler
   int nbx = 0, nby = 0, nbz = 0;
   long long nblocks = 0;
@@ -249,12 +274,8 @@ struct pdfs_ctx {
   float mlp_thr = 0.0f;          // its decision threshold on the logit
   bool loaded = false, has_mask = false;
   int last_prec = -1;      // which working field holds the last result
-  cudaEvent_t e0 = nullptr, e1 = nullptr, k0 = nullptr, k1 = nullptr, q0 = nullptr, q1 = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr, k0 = nullptr, k1 = nullptr, q0 = nullptr, q1 = nullptr;  // hd.ev
   cudaEvent_t r0 = nullptr, r1 = nullptr;  // around a whole pdfs_ctx_run
-  // load / store pipeline: slab copies on st, layout kernels on st2
-  cudaStream_t st2 = nullptr;
-  static constexpr int kSlabs = 32;
-  cudaEvent_t slab_ev[kSlabs + 1] = {};
   double kern_ms = 0.0;  // accumulated sweep-kernel time since the last reset
   int launches = 0;      // kernels launched since the last reset
 };

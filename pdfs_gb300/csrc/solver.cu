@@ -566,9 +566,7 @@ void cache_release(int dev) {
 }  // namespace
 
 // A block of at least `bytes` (a cached one of at most 1/8 more, else new).
-template <class P>
-static cudaError_t ctx_malloc(pdfs_ctx *c, P **out, size_t bytes) {
-  const int dev = c->dev;
+cudaError_t pdfs::block_take(int dev, void **out, size_t bytes) {
   if (dev >= 0 && dev < 64) {
     BlockCache &bc = block_cache();
     std::lock_guard<std::mutex> lk(bc.m);
@@ -580,7 +578,7 @@ static cudaError_t ctx_malloc(pdfs_ctx *c, P **out, size_t bytes) {
         best = (int)i;
     }
     if (best >= 0) {
-      *out = reinterpret_cast<P *>(bc.blocks[best].p);
+      *out = bc.blocks[best].p;
       bc.held[dev] -= bc.blocks[best].bytes;
       bc.blocks[best] = bc.blocks.back();
       bc.blocks.pop_back();
@@ -594,14 +592,13 @@ static cudaError_t ctx_malloc(pdfs_ctx *c, P **out, size_t bytes) {
     cache_release(dev);
     e = cudaMalloc(&p, bytes);
   }
-  *out = reinterpret_cast<P *>(p);
+  *out = p;
   return e;
 }
 // Returns an idle block of `bytes` to the cache (or to the device when the
 // cache is full).
-static void ctx_free(pdfs_ctx *c, void *p, size_t bytes) {
+void pdfs::block_give(int dev, void *p, size_t bytes) {
   if (!p) return;
-  const int dev = c->dev;
   if (dev >= 0 && dev < 64) {
     const size_t cap = cache_cap(dev);
     BlockCache &bc = block_cache();
@@ -615,6 +612,86 @@ static void ctx_free(pdfs_ctx *c, void *p, size_t bytes) {
   cudaFree(p);
 }
 
+// Idle sets of handles, at most kMostHandles a process (a batch of 32 grids takes
+// 33): given back with the block cache.  A 37 x 22 x 19 sweep through the one-call
+// API took 707 us making and destroying its own, 373 with the pool;
+// a batch of 32 grids to 160^3 16.4 and 15.5 ms.
+namespace {
+constexpr size_t kMostHandles = 64;
+struct HandlePool {
+  std::mutex m;
+  std::vector<std::pair<int, Handles>> idle;
+};
+HandlePool &handle_pool() {
+  static HandlePool *hp = new HandlePool();  // never destroyed, as the block cache
+  return *hp;
+}
+void handles_destroy(Handles &h) {
+  for (cudaEvent_t ev : h.ev)
+    if (ev) cudaEventDestroy(ev);
+  for (cudaEvent_t ev : h.slab_ev)
+    if (ev) cudaEventDestroy(ev);
+  if (h.pinned) cudaFreeHost(h.pinned);
+  if (h.st2) cudaStreamDestroy(h.st2);
+  if (h.st) cudaStreamDestroy(h.st);
+  h = Handles();
+}
+void handles_release(int dev) {
+  std::vector<Handles> drop;
+  {
+    HandlePool &hp = handle_pool();
+    std::lock_guard<std::mutex> lk(hp.m);
+    for (size_t i = 0; i < hp.idle.size();) {
+      if (hp.idle[i].first == dev) {
+        drop.push_back(hp.idle[i].second);
+        hp.idle[i] = hp.idle.back();
+        hp.idle.pop_back();
+      } else {
+        ++i;
+      }
+    }
+  }
+  for (Handles &h : drop) handles_destroy(h);
+}
+}  // namespace
+
+cudaError_t pdfs::handles_take(int dev, Handles *h) {
+  {
+    HandlePool &hp = handle_pool();
+    std::lock_guard<std::mutex> lk(hp.m);
+    for (size_t i = hp.idle.size(); i-- > 0;)
+      if (hp.idle[i].first == dev) {
+        *h = hp.idle[i].second;
+        hp.idle[i] = hp.idle.back();
+        hp.idle.pop_back();
+        return cudaSuccess;
+      }
+  }
+  cudaError_t e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaHostAlloc(&h->pinned, kPinned, cudaHostAllocDefault);
+  for (cudaEvent_t &ev : h->ev)
+    if (e == cudaSuccess) e = cudaEventCreate(&ev);
+  if (e != cudaSuccess) handles_destroy(*h);
+  return e;
+}
+
+void pdfs::handles_give(int dev, Handles *h) {
+  if (!h->st) return;
+  bool ok = true;
+  if (h->st2) ok = cudaStreamSynchronize(h->st2) == cudaSuccess && ok;
+  ok = cudaStreamSynchronize(h->st) == cudaSuccess && ok;
+  if (ok) {
+    HandlePool &hp = handle_pool();
+    std::lock_guard<std::mutex> lk(hp.m);
+    if (hp.idle.size() < kMostHandles) {
+      hp.idle.emplace_back(dev, *h);
+      *h = Handles();
+      return;
+    }
+  }
+  handles_destroy(*h);
+}
+
 extern "C" int pdfs_release_cached(int device) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) {
@@ -624,6 +701,7 @@ extern "C" int pdfs_release_cached(int device) {
   if (device < 0 || device >= ndev) return PDFS_ERR_INVALID;
   CK(cudaSetDevice(device));
   cache_release(device);
+  handles_release(device);
   return PDFS_OK;
 }
 
@@ -755,7 +833,12 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
   };
   cudaError_t e;
   if ((e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->dev)) != cudaSuccess) return fail(e);
-  if ((e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
+  if ((e = handles_take(c->dev, &c->hd)) != cudaSuccess) return fail(e);
+  c->st = c->hd.st;
+  c->hstat = reinterpret_cast<DevStatus *>(c->hd.pinned);
+  static_assert(sizeof(DevStatus) <= kPinned, "status copy");
+  cudaEvent_t *const evs[8] = {&c->e0, &c->e1, &c->k0, &c->k1, &c->q0, &c->q1, &c->r0, &c->r1};
+  for (int i = 0; i < 8; ++i) *evs[i] = c->hd.ev[i];
   mark("stream");
   // Host tables first, then every device buffer of the context carved from
   // one allocation (a batch creates hundreds of contexts: one allocation, or
@@ -895,7 +978,7 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
   {
     size_t total = 0;
     for (auto &r : plan) total += (r.second + 255) & ~(size_t)255;  // 256-byte aligned pieces
-    if ((e = ctx_malloc(c, &c->arena, total)) != cudaSuccess) return fail(e);
+    if ((e = block_take(c->dev, (void **)&c->arena, total)) != cudaSuccess) return fail(e);
     c->arena_bytes = total;
     char *p = reinterpret_cast<char *>(c->arena);
     for (auto &r : plan) {
@@ -904,7 +987,6 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
     }
   }
   mark("allocation");
-  if ((e = cudaHostAlloc(&c->hstat, sizeof(DevStatus), cudaHostAllocDefault)) != cudaSuccess) return fail(e);
   GodPerm64 perm[6];
   fill_perm(*g, perm);
   if ((e = cudaMemcpyAsync(c->kperm, perm, sizeof perm, cudaMemcpyHostToDevice, c->st)) != cudaSuccess) return fail(e);
@@ -945,14 +1027,6 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
   if (c->u64) fill_padding(c->u64, c->L64, c->g, c->sms, c->st);
   if (c->u32) fill_padding(c->u32, c->L32, c->g, c->sms, c->st);
   if ((e = cudaMemsetAsync(c->fmask, 0, c->M.words * 4, c->st)) != cudaSuccess) return fail(e);
-  if ((e = cudaEventCreate(&c->e0)) != cudaSuccess) return fail(e);
-  if ((e = cudaEventCreate(&c->e1)) != cudaSuccess) return fail(e);
-  if ((e = cudaEventCreate(&c->k0)) != cudaSuccess) return fail(e);
-  if ((e = cudaEventCreate(&c->k1)) != cudaSuccess) return fail(e);
-  if ((e = cudaEventCreate(&c->q0)) != cudaSuccess) return fail(e);
-  if ((e = cudaEventCreate(&c->q1)) != cudaSuccess) return fail(e);
-  if ((e = cudaEventCreate(&c->r0)) != cudaSuccess) return fail(e);
-  if ((e = cudaEventCreate(&c->r1)) != cudaSuccess) return fail(e);
   if ((e = cudaStreamSynchronize(c->st)) != cudaSuccess) return fail(e);
   if (verbose(o)) {
     const auto t_end = std::chrono::steady_clock::now();
@@ -973,23 +1047,11 @@ extern "C" void pdfs_ctx_destroy(pdfs_ctx *c) {
   if (!c) return;
   cudaSetDevice(c->dev);
   // every block is idle before it goes back to the cache
-  if (c->st2) cudaStreamSynchronize(c->st2);
+  if (c->hd.st2) cudaStreamSynchronize(c->hd.st2);
   if (c->st) cudaStreamSynchronize(c->st);
-  ctx_free(c, c->arena, c->arena_bytes);
-  ctx_free(c, c->stage, c->stage_bytes);
-  if (c->hstat) cudaFreeHost(c->hstat);
-  if (c->e0) cudaEventDestroy(c->e0);
-  if (c->e1) cudaEventDestroy(c->e1);
-  if (c->k0) cudaEventDestroy(c->k0);
-  if (c->k1) cudaEventDestroy(c->k1);
-  if (c->q0) cudaEventDestroy(c->q0);
-  if (c->q1) cudaEventDestroy(c->q1);
-  if (c->r0) cudaEventDestroy(c->r0);
-  if (c->r1) cudaEventDestroy(c->r1);
-  for (cudaEvent_t ev : c->slab_ev)
-    if (ev) cudaEventDestroy(ev);
-  if (c->st2) cudaStreamDestroy(c->st2);
-  if (c->st) cudaStreamDestroy(c->st);
+  block_give(c->dev, c->arena, c->arena_bytes);
+  block_give(c->dev, c->stage, c->stage_bytes);
+  handles_give(c->dev, &c->hd);
   cudaGetLastError();
   delete c;
 }
@@ -1001,10 +1063,10 @@ static int ensure_stage(pdfs_ctx *c) {
   const size_t b = ref_nodes(c->g) * 9;
   if (c->stage_bytes >= b) return PDFS_OK;
   if (c->stage) CK(cudaStreamSynchronize(c->st));  // the old stage is idle
-  ctx_free(c, c->stage, c->stage_bytes);
+  block_give(c->dev, c->stage, c->stage_bytes);
   c->stage = nullptr;
   c->stage_bytes = 0;
-  CK(ctx_malloc(c, &c->stage, b));
+  CK(block_take(c->dev, (void **)&c->stage, b));
   c->stage_bytes = b;
   return PDFS_OK;
 }
@@ -1015,14 +1077,14 @@ static int ensure_stage(pdfs_ctx *c) {
 static int slab_planes(const pdfs_grid &g) {
   const int planes = g.nz + 2;
   if (ref_nodes(g) * 8 < (256u << 20)) return planes;
-  return std::max(16, (planes + pdfs_ctx::kSlabs - 1) / pdfs_ctx::kSlabs);
+  return std::max(16, (planes + kSlabs - 1) / kSlabs);
 }
 
 // The pipeline's second stream and slab events, made on first use.
 static int ensure_pipeline(pdfs_ctx *c) {
-  if (c->st2) return PDFS_OK;
-  CK(cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking));
-  for (cudaEvent_t &ev : c->slab_ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  for (cudaEvent_t &ev : c->hd.slab_ev)
+    if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  if (!c->hd.st2) CK(cudaStreamCreateWithFlags(&c->hd.st2, cudaStreamNonBlocking));
   return PDFS_OK;
 }
 
@@ -1033,7 +1095,7 @@ static double ms_between(cudaEvent_t a, cudaEvent_t b) {
 }
 
 // Host -> device.  The mask goes first (the cap bounds need it), then the
-// field in z-slabs on c->st; c->st2 packs each slab as it lands and takes the
+// field in z-slabs on c->st; c->hd.st2 packs each slab as it lands and takes the
 // cap bounds of the 8^3 blocks whose planes are all packed, so that only the
 // last slab's kernels trail the copies.
 static int load_impl(pdfs_ctx *c, const double *field, const uint8_t *frozen, double *ms_h2d) {
@@ -1054,7 +1116,7 @@ static int load_impl(pdfs_ctx *c, const double *field, const uint8_t *frozen, do
   const int planes = g.nz + 2, per = dev_field ? planes : slab_planes(g);
   const bool pipe = per < planes;  // else every step runs on c->st
   if (pipe && (s = ensure_pipeline(c))) return s;
-  cudaStream_t ks = pipe ? c->st2 : c->st;  // the layout kernels' stream
+  cudaStream_t ks = pipe ? c->hd.st2 : c->st;  // the layout kernels' stream
   auto handoff = [&](cudaEvent_t ev) -> cudaError_t {  // ks waits for the copies issued so far
     if (!pipe) return cudaSuccess;
     cudaError_t e = cudaEventRecord(ev, c->st);
@@ -1069,7 +1131,7 @@ static int load_impl(pdfs_ctx *c, const double *field, const uint8_t *frozen, do
     if (!dev_mask) {
       m = (const uint8_t *)c->stage + n * 8;
       CK(cudaMemcpyAsync((void *)m, frozen, n, cudaMemcpyHostToDevice, c->st));
-      CK(handoff(c->slab_ev[pdfs_ctx::kSlabs]));
+      CK(handoff(c->hd.slab_ev[kSlabs]));
     }
     k_pack_mask<<<(unsigned)(((long long)g.ny * g.nz + kRowWarps - 1) / kRowWarps), 32 * kRowWarps, 0, ks>>>(
         m, c->fmask, c->M, g.nx, g.ny, g.nz);
@@ -1081,7 +1143,7 @@ static int load_impl(pdfs_ctx *c, const double *field, const uint8_t *frozen, do
     if (!dev_field) {
       CK(cudaMemcpyAsync((char *)c->stage + z0 * plane * 8, field + z0 * plane, (size_t)(z1 - z0) * plane * 8,
                          cudaMemcpyHostToDevice, c->st));
-      CK(handoff(c->slab_ev[k]));
+      CK(handoff(c->hd.slab_ev[k]));
     }
     dim3 grid(g.ny + 2, z1 - z0);
     k_pack<double><<<grid, 128, 0, ks>>>(src, c->in64, g.nx, g.ny, c->L64, z0);
@@ -1616,7 +1678,7 @@ extern "C" int pdfs_ctx_run(pdfs_ctx *c, pdfs_stats *stats) {
 }
 
 // Device -> host: c->st converts the result to the reference layout slab by
-// slab, c->st2 copies each converted slab out.
+// slab, c->hd.st2 copies each converted slab out.
 static int store_impl(pdfs_ctx *c, double *field, double *ms_d2h) {
   if (!c || !field || c->last_prec < 0) return PDFS_ERR_INVALID;
   CK(cudaSetDevice(c->dev));
@@ -1632,7 +1694,7 @@ static int store_impl(pdfs_ctx *c, double *field, double *ms_d2h) {
   const int planes = g.nz + 2, per = dev ? planes : slab_planes(g);
   const bool pipe = per < planes;  // else the copy runs on c->st
   if (pipe && (s = ensure_pipeline(c))) return s;
-  cudaStream_t cs = pipe ? c->st2 : c->st;  // the copies' stream
+  cudaStream_t cs = pipe ? c->hd.st2 : c->st;  // the copies' stream
   CK(cudaEventRecord(c->e0, c->st));
   const uint32_t *fm = c->has_mask ? c->fmask : nullptr;
   for (int z0 = 0, k = 0; z0 < planes; z0 += per, ++k) {
@@ -1648,16 +1710,16 @@ static int store_impl(pdfs_ctx *c, double *field, double *ms_d2h) {
     CK(cudaGetLastError());
     if (!dev) {
       if (pipe) {
-        CK(cudaEventRecord(c->slab_ev[k], c->st));
-        CK(cudaStreamWaitEvent(cs, c->slab_ev[k], 0));
+        CK(cudaEventRecord(c->hd.slab_ev[k], c->st));
+        CK(cudaStreamWaitEvent(cs, c->hd.slab_ev[k], 0));
       }
       CK(cudaMemcpyAsync(field + z0 * plane, (char *)c->stage + z0 * plane * 8, (size_t)(z1 - z0) * plane * 8,
                          cudaMemcpyDeviceToHost, cs));
     }
   }
   if (pipe) {
-    CK(cudaEventRecord(c->slab_ev[pdfs_ctx::kSlabs], cs));
-    CK(cudaStreamWaitEvent(c->st, c->slab_ev[pdfs_ctx::kSlabs], 0));
+    CK(cudaEventRecord(c->hd.slab_ev[kSlabs], cs));
+    CK(cudaStreamWaitEvent(c->st, c->hd.slab_ev[kSlabs], 0));
   }
   CK(cudaEventRecord(c->e1, c->st));
   CK(cudaStreamSynchronize(c->st));
