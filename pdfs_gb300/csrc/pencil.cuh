@@ -29,7 +29,8 @@
 //   * pencils are taken by ticket in wavefront order, so an upwind pencil is
 //     always running or done; every wait is bounded (SweepArgs::wait_cycles)
 //     and ends in DEV_ERR_TIMEOUT plus the abort flag, never in a hang.
-// Sweeps with a block mask or block-change output run on bricks instead.
+// Sweeps with a block mask or block-change output run on bricks instead, and so do
+// the plain ones but for pairs and mixed on large grids and batches (pick_tiles).
 #pragma once
 #include "sweep.cuh"
 

@@ -1346,9 +1346,9 @@ static int run_sweep(pdfs_ctx *c, int which, int sn, const uint8_t *active, unsi
     }
     return PDFS_OK;
   }
-  // pencils sweep unmasked sweeps; a block mask or block-change output goes to bricks
-  // (pencils that recorded block changes measured no faster: 37.4 against 36.9 ms
-  // for the 8 recording sweeps of the 768^3 headline solve)
+  // pencil tiles: plain sweeps by pick_tiles' rule, on bricks or pencils; a block mask
+  // or block-change output goes to the masked bricks (pencils that recorded block
+  // changes measured no faster: 37.4 against 36.9 ms for 8 recording 768^3 sweeps)
   const bool pencil = ts.pencil && !active && !blk_chg;
   const pdfs_ctx::Plain &pl = f32 ? c->plain32 : c->plain64;
   if (ts.bz == 0 || (pencil && !pl.b)) CK(cudaMemsetAsync(c->progress, 0, (size_t)L.ncx * L.ncy * L.ty * 4, c->st));
