@@ -506,8 +506,9 @@ extern "C" int pdfs_solve_batch(int n, const pdfs_grid *grids, double *const *fi
   for (int g = 0; g < n; ++g) all[g] = g;
   const int max_sweeps = o.max_sweeps > 0 ? o.max_sweeps : 100000;
   if (o.precision == PDFS_PREC_FP64) {
-    for (auto *c : ctx)
-      BQ(cudaMemcpyAsync(c->u64, c->in64, c->L64.elems * 8, cudaMemcpyDeviceToDevice, c->st));
+    for (auto *c : ctx) {
+      if ((rc = ctx_fp64_start(c))) return cleanup(rc);
+    }
     for (auto *c : ctx) BQ(cudaStreamSynchronize(c->st));
     rc = (pen64 ? batch_phase_pencils : batch_phase)(B, ctx, all, 1, o.tol, max_sweeps, st, &kms64, &launches);
     for (auto *c : ctx) c->last_prec = 1;
