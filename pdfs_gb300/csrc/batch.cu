@@ -40,7 +40,6 @@ struct BatchState {
   int *d_err = nullptr;                 // [4]
   int *h_err = nullptr;                 // pinned
   int *d_ticket = nullptr;
-  int *d_done = nullptr;   // pencil rounds: [grid * 8 + sweep] pencils finished
   int *d_round = nullptr;  // pencil rounds: rounds run in this phase
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
@@ -281,6 +280,8 @@ int batch_phase_pencils(BatchState &B, std::vector<pdfs_ctx *> &ctx, const std::
     args[g].ticket = B.d_ticket;
     const Layout &L = f32 ? c->L32 : c->L64;
     BK(encode_pencil_maps(which, args[g], L, &maps[3 * (size_t)g]));
+    // the pencils' flags: below every epoch of this phase
+    BK(cudaMemsetAsync(c->progress, 0, sizeof(int) * L.ncx * L.ncy, B.st));
   }
   BK(cudaMemcpyAsync(B.d_args, args.data(), sizeof(SweepArgs) * n, cudaMemcpyHostToDevice, B.st));
   BK(cudaMemcpyAsync(B.d_maps, maps.data(), sizeof(CUtensorMap) * 3 * n, cudaMemcpyHostToDevice, B.st));
@@ -302,7 +303,7 @@ int batch_phase_pencils(BatchState &B, std::vector<pdfs_ctx *> &ctx, const std::
         for (int lc : ord[g]) tickets.push_back(make_int2(g * 8 + s, lc));
     if (tickets.empty()) return PDFS_OK;
     BK(cudaMemcpyAsync(B.d_tickets, tickets.data(), sizeof(int2) * tickets.size(), cudaMemcpyHostToDevice, B.st));
-    BatchDesc desc{(int)tickets.size(), B.d_tickets, B.d_args, B.d_maps, n, B.d_done, B.d_round};
+    BatchDesc desc{(int)tickets.size(), B.d_tickets, B.d_args, B.d_maps, n, B.d_round};
     BK(cudaMemcpyAsync(B.d_desc, &desc, sizeof(desc), cudaMemcpyHostToDevice, B.st));
     return PDFS_OK;
   };
@@ -317,7 +318,6 @@ int batch_phase_pencils(BatchState &B, std::vector<pdfs_ctx *> &ctx, const std::
   a0.maxchg = B.d_chg;
   a0.batch = B.d_desc;
   auto enqueue_round = [&]() -> int {
-    BK(cudaMemsetAsync(B.d_done, 0, sizeof(int) * 8 * n, B.st));
     BK(cudaMemsetAsync(B.d_ticket, 0, 4, B.st));
     int grid = 0;
     BK(launch_pencil_round(which, arith, iso, a0, max_ticks, B.sms, B.st, &grid));
@@ -481,7 +481,6 @@ extern "C" int pdfs_solve_batch(int n, const pdfs_grid *grids, double *const *fi
     want(&B.d_chg, sizeof(unsigned long long) * 8 * n);
     want(&B.d_err, 16);
     want(&B.d_ticket, 16);
-    want(&B.d_done, sizeof(int) * 8 * n);
     want(&B.d_round, 16);
     for (auto &r : plan) B.block_bytes += r.second;
     BQ(block_take(B.dev, &B.block, B.block_bytes));

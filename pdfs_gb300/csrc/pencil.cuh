@@ -98,10 +98,15 @@ __device__ __forceinline__ const SweepArgs &pc_args(const SweepArgs &a0) {
 }
 
 // BATCH: one launch runs a whole round -- the 8 orderings of every grid of a
-// batch (BatchDesc).  A ticket names (grid, sweep, pencil); sweep s of a grid
-// starts once every pencil of its sweep s - 1 has finished (a per-(grid,
-// sweep) counter, bounded wait), and tickets list every grid's sweep s before
-// any grid's sweep s + 1, so every wait is on smaller tickets.
+// batch (BatchDesc).  A ticket names (grid, sweep, pencil); a pencil of sweep s
+// starts once it and its four face neighbours have finished sweep s - 1 (an epoch
+// flag each, bounded wait): their values are its old values, its mailboxes have
+// been read, and a neighbour cannot be two sweeps ahead.  Tickets list every grid's
+// sweep s before any grid's sweep s + 1, so every wait is on smaller tickets.  A
+// round is bound by the chain of its largest grids' 8 sweeps: waiting for a grid's
+// whole sweep s - 1 instead made that chain 8 full sweeps long (32 grids of 32 to
+// 160 nodes a side: 17.3 ms, this 16.3; 12 of 24 to 154: 6.4 and 4.9; 7 of 24 to 171:
+// 4.9 and 3.6).
 template <class T, int MODE, int ARITH, bool ISO, bool BATCH = false>
 __global__ void __launch_bounds__(PcGeo<T>::NT) pc_sweep_kernel(const __grid_constant__ CUtensorMap tm_u,
                                                                const __grid_constant__ CUtensorMap tm_mask,
@@ -175,31 +180,33 @@ __global__ void __launch_bounds__(PcGeo<T>::NT) pc_sweep_kernel(const __grid_con
           S.ticket = a0.ticket;
           S.maxchg = reinterpret_cast<unsigned long long *>(a0.maxchg) + (size_t)sw * a0.batch->ngrid + g;
           s_maps = a0.batch->maps + 3 * g;
-          // the grid's previous sweep must be complete: its stores, then its count (release)
-          if (sw > 0) {
-            const int *cnt = a0.batch->done + cur_gs - 1;
-            const int need = S.ncx * S.ncy;
-            if (ld_acquire_gpu(cnt) < need) {
-              const long long t0 = cycles();
-              unsigned nap = 32;
-              while (ld_acquire_gpu(cnt) < need) {
-                if (s_abort || *(volatile int *)(a0.err + 1)) {
-                  s_abort = 1;
-                  break;
-                }
-                if (cycles() - t0 > S.wait_cycles) {
-                  raise_timeout(S, -1, &s_abort);
-                  break;
-                }
-                __nanosleep(nap);
-                nap = min(nap * 2, 256u);
-              }
-            }
-          }
         }
         __syncthreads();
-        if (s_abort) break;
       }
+      // my pencil and its face neighbours: lanes 0 .. 4 wait for their flags
+      if (warp == 0 && (cur_gs & 7) > 0) {
+        const int wx = s_lc % a.ncx, wy = s_lc / a.ncx;
+        const int fx = (a.sx > 0 ? wx : a.ncx - 1 - wx) + (lane == 1) - (lane == 2);
+        const int fy = (a.sy > 0 ? wy : a.ncy - 1 - wy) + (lane == 3) - (lane == 4);
+        const bool mine = lane < 5 && fx >= 0 && fx < a.ncx && fy >= 0 && fy < a.ncy;
+        const int *flag = a.prog + (mine ? fy * a.ncx + fx : 0);
+        const long long t0 = cycles();
+        unsigned nap = 32;
+        while (!__all_sync(0xffffffffu, !mine || ld_acquire_gpu(flag) >= a.epoch - 1)) {
+          if (__any_sync(0xffffffffu, s_abort || *(volatile int *)(a.err + 1))) {
+            if (lane == 0) s_abort = 1;
+            break;
+          }
+          if (__any_sync(0xffffffffu, cycles() - t0 > a.wait_cycles)) {
+            if (lane == 0) raise_timeout(a, -1, &s_abort);
+            break;
+          }
+          __nanosleep(nap);
+          nap = min(nap * 2, 256u);
+        }
+      }
+      __syncthreads();
+      if (s_abort) break;
     }
     const int sxd = a.sx, syd = a.sy, szd = a.sz;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
@@ -236,7 +243,7 @@ __global__ void __launch_bounds__(PcGeo<T>::NT) pc_sweep_kernel(const __grid_con
       unsigned nap = 0;
       bool failed = false;
       // a round's earlier sweep was written by other CTAs of this launch:
-      // order the acquire of its count before these async-proxy reads
+      // order the acquire of its flags before these async-proxy reads
       if constexpr (BATCH) fence_proxy_async_global();
       for (;;) {
         int moved = 0;
@@ -461,11 +468,10 @@ __global__ void __launch_bounds__(PcGeo<T>::NT) pc_sweep_kernel(const __grid_con
     }
     __syncthreads();
     if (s_abort) break;
-    if constexpr (BATCH) {  // the pencil is done: count it (release)
-      if (tid == 0) {
-        __threadfence();
-        atomicAdd(a0.batch->done + cur_gs, 1);
-      }
+    // the pencil is done.  The barrier orders every thread's stores before this
+    // thread's GPU-scope fence, which orders them before the flag.
+    if constexpr (BATCH) {
+      if (tid == 0) publish_gpu(a.prog + col, epoch);
     }
   }
   // the CTA's max change -> the grid's counter (one atomic per warp)

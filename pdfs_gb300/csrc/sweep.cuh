@@ -160,9 +160,9 @@ struct BatchDesc {
   const SweepArgs *args;    // per grid (sx/sy/sz are taken from the launch)
   const CUtensorMap *maps;  // per grid: field, cap, mask
   // Pencil rounds (pencil.cuh): one launch runs all 8 orderings of a round
-  // for every grid; sweep s of a grid starts once its sweep s - 1 is done.
+  // for every grid; a pencil's sweep s starts once its neighbourhood's sweep s - 1 is
+  // done (the grids' prog words hold each pencil's last epoch).
   int ngrid;                // grids in args; the change words are [sweep][grid]
-  int *done;                // [grid * 8 + sweep]: pencils finished this round
   const int *round;         // rounds run before this one (mailbox epochs advance 8 per round)
 };
 
@@ -342,6 +342,15 @@ __device__ __forceinline__ T cap_value(const T *p) {
     return p_from_double(__ldg(p));
   else
     return __ldg(p);
+}
+
+// A brick's completion: the CTA barrier before it orders every thread's
+// stores before thread 0's acquire-release fence at GPU scope, which orders
+// them before the relaxed flag store (the fence-then-relaxed-store pattern of
+// CUTLASS's arrival barriers).
+__device__ __forceinline__ void publish_gpu(int *p, int v) {
+  asm volatile("fence.acq_rel.gpu;\n" ::: "memory");
+  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
 
 // A node's change as a kernel accumulates it: relative for FP32, absolute

@@ -156,15 +156,6 @@ struct T3Desc {
   unsigned act, upx, upy, upz;
 };
 
-// A brick's completion: the CTA barrier before it orders every thread's
-// stores before thread 0's acquire-release fence at GPU scope, which orders
-// them before the relaxed flag store (the fence-then-relaxed-store pattern of
-// CUTLASS's arrival barriers).
-__device__ __forceinline__ void publish_gpu(int *p, int v) {
-  asm volatile("fence.acq_rel.gpu;\n" ::: "memory");
-  asm volatile("st.relaxed.gpu.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
-}
-
 // The brick's BX x BY columns are listed by diagonal d = lx + ly (then by
 // ly).  Column (lx, ly) holds a node of level L
 // for L - lx - ly in [0, BZ), so a warp whose 32 columns span diagonals
