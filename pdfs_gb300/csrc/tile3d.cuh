@@ -56,6 +56,7 @@
 // and returns.
 #pragma once
 #include "god64.cuh"
+#include "oct_wait.h"
 #include "sweep.cuh"
 
 namespace pdfs {
@@ -243,12 +244,7 @@ __device__ __forceinline__ void t3_next(const SweepArgs &a, int ntile, T3Desc &d
         if (lane == 4 && bj < nty - 1) n = tile + ntx;
         if (lane == 5 && bk > 0) n = tile - ntx * nty;
         if (lane == 6 && bk < ntz - 1) n = tile + ntx * nty;
-        int need = -1;
-        if (n >= 0) {
-          const unsigned tb = __ldg(a.oct_tbits + n);
-          for (int j = osw - 1; j >= 0 && need < 0; --j)
-            if (((a.oct_full >> j) & 1u) || ((tb >> ((a.oct_first + j) % 8)) & 1u)) need = j;
-        }
+        const int need = n >= 0 ? oct_latest(osw, a.oct_first, a.oct_full, a.oct_tbits, n) : -1;
         // (the CTA's current brick may be among them: looked at here, waited for later)
         if (need >= 0 && ld_acquire_gpu(a.tflag + n) < a.epoch + need) {
           wait_flag = n;
