@@ -6,8 +6,10 @@
 // over the pencils of every grid still sweeping: the ticket table lists
 // (grid, sweep, pencil) triples, every grid's sweep s before any grid's sweep
 // s + 1 and each grid's pencils in wavefront order, and a pencil of sweep s
-// starts once its grid's sweep s - 1 is complete -- so every wait is on a
-// smaller ticket held by a running CTA.  On column tiles each sweep is one
+// starts once it and its four face neighbours have finished sweep s - 1 (an epoch
+// flag per pencil: zero at the start of a phase, and a round's epochs lie above all
+// earlier ones, 8 a round) -- so every wait is on a smaller ticket held by a running
+// CTA.  On column tiles each sweep is one
 // launch over (grid, column) pairs.  Rounds after the first replay a captured
 // CUDA graph; after each round the per-grid, per-sweep changes come back in
 // one copy, and converged grids leave the ticket table.
@@ -442,6 +444,9 @@ extern "C" int pdfs_solve_batch(int n, const pdfs_grid *grids, double *const *fi
   BatchState B;
   B.n = n;
   auto cleanup = [&](int s) {
+    // a call that failed may leave memsets and a round queued on the contexts' memory,
+    // and a context's memory is another thread's as soon as the context is destroyed
+    if (B.st) cudaStreamSynchronize(B.st);
     for (auto *c : ctx) pdfs_ctx_destroy(c);
     if (stats) {
       const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
