@@ -362,8 +362,9 @@ __global__ void __launch_bounds__(256) k_block_capmin(const double *__restrict__
   __syncthreads();
   const int bx = wx * 4 + (int)threadIdx.x;
   if (threadIdx.x < 4 && bx < nbx) {
+    m = s_m[0][threadIdx.x];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 1; j < 8; ++j)
       if (dkey(s_m[j][threadIdx.x]) < dkey(m)) m = s_m[j][threadIdx.x];
     const long long b = ((long long)bz * nby + by) * nbx + bx;
     b64[b] = m;
@@ -1862,6 +1863,17 @@ extern "C" int pdfs_ctx_orderings(pdfs_ctx *c, uint8_t *orderings) {
     buf = c->bact;
   }
   CK(cudaMemcpyAsync(orderings, buf, (size_t)c->nblocks, cudaMemcpyDefault, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  return PDFS_OK;
+}
+
+// For the tests (not in pdfs.h): the replace-update's cap bounds, a value per 8^3
+// block, as the last load left them.
+extern "C" int pdfs_test_caps(pdfs_ctx *c, double *caps64, float *caps32) {
+  if (!c || !c->loaded || !c->bcap64 || !caps64 || !caps32) return PDFS_ERR_INVALID;
+  CK(cudaSetDevice(c->dev));
+  CK(cudaMemcpyAsync(caps64, c->bcap64, (size_t)c->nblocks * 8, cudaMemcpyDefault, c->st));
+  CK(cudaMemcpyAsync(caps32, c->bcap32, (size_t)c->nblocks * 4, cudaMemcpyDefault, c->st));
   CK(cudaStreamSynchronize(c->st));
   return PDFS_OK;
 }
