@@ -274,6 +274,7 @@ struct pdfs_ctx {
   float mlp_thr = 0.0f;          // its decision threshold on the logit
   bool loaded = false, has_mask = false;
   int last_prec = -1;      // which working field holds the last result
+  bool u32_set = false;    // the FP32 field has been written (a new context's is not)
   cudaEvent_t e0 = nullptr, e1 = nullptr, k0 = nullptr, k1 = nullptr, q0 = nullptr, q1 = nullptr;  // hd.ev
   cudaEvent_t r0 = nullptr, r1 = nullptr;  // around a whole pdfs_ctx_run
   double kern_ms = 0.0;  // accumulated sweep-kernel time since the last reset

@@ -1459,6 +1459,7 @@ int pdfs::ctx_widen(pdfs_ctx *c) {
 
 int pdfs::ctx_narrow(pdfs_ctx *c) {  // FP64 input -> FP32 working field
   const pdfs_grid &g = c->g;
+  c->u32_set = true;
   if (c->L32.zc) return zc_fill<float>(c, c->u32, c->L32, false);
   k_convert<double, float><<<row_blocks(g), 32 * kRowWarps, 0, c->st>>>(c->in64, c->L64, c->u32, c->L32, g.nx, g.ny,
                                                                          g.nz);
@@ -1856,6 +1857,11 @@ extern "C" int pdfs_ctx_orderings(pdfs_ctx *c, uint8_t *orderings) {
   if (!c || !c->loaded || !c->u32 || !c->omask || !orderings || c->last_prec < 0) return PDFS_ERR_INVALID;
   CK(cudaSetDevice(c->dev));
   const uint8_t *buf = c->omask;
+  if (!c->u32_set) {  // FP64 sweeps alone: no node has an FP32 value, so none accepts an ordering
+    k_fill<float><<<2 * c->sms, 256, 0, c->st>>>(c->u32, c->L32.elems, INFINITY);
+    CK(cudaGetLastError());
+    c->u32_set = true;
+  }
   CK(octant_mask(c->u32, c->L32, c->has_mask ? c->fmask : nullptr, c->M, c->g, kOctSlack32, INFINITY, c->nbx,
                  c->nby, c->nbz, c->omask, c->st));
   if (kOctDilate) {  // the polish's widened masks: bit sn of a block or of a face neighbour
