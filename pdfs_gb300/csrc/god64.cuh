@@ -11,14 +11,16 @@
 // (P. W. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", IBM J. Res. Dev. 34, 1990: with y = RN(1/b), q within
 // an ulp of a/b and r = a - b q exact, RN(q + r y) = RN(a/b)), and a square root
-// starts from an FP32 reciprocal root refined to 45 bits in FP32: 61 and 25
-// FP64 operations an update.  A node with three terms is mostly known to have them
-// before its two-term solution is: 44 and 16.  Rounding by rounding, god64_ref is
-// god_ref64.
-// One warp, a three-term update: 3583 cycles against 6631 (reference), 1480 against
-// 3950 (fast); 4585 and 2043 with the two-term solution always first (a 384^3
-// sweep, 8 x 8 x 16 bricks: 10.1 -> 8.8 ms reference, 4.56 -> 4.04 fast; 64^3, where a
-// level's lanes rarely agree, even).
+// starts from an FP32 reciprocal root refined to 45 bits in FP32 (the series of
+// (1 - e)^(-1/2) to second order, e the exact residual): 61 and 29 FP64 operations an
+// update.  A node with three terms is mostly known to have them without its two-term
+// solution: 44 and 18.  Rounding by rounding, god64_ref is god_ref64 and god64_fast is
+// god_fast64: bricks give the bits of columns, pencils and batches.
+// A 384^3 sweep, 8 x 8 x 16 bricks: 8.9 ms reference and 4.4 fast, on pencils with the
+// plain solvers 18.7 and 10.4; with the two-term solution always first 10.1
+// (reference).  The fast one takes 4.5 with three_terms as its test too; 4.0 with roots
+// to within an ulp and products with reciprocals instead of divisions, but then its
+// bits are not the other tiles'.  64^3: 0.54 and 0.34 (pencils 1.35 and 0.82).
 //
 // They take finite or +inf non-negative values; anything else (negative
 // values, NaN) goes to the plain solvers.
@@ -77,12 +79,10 @@ __device__ __forceinline__ double sqrt_core(double m) {
   return __fma_rn(__fma_rn(-s, s, m), hr, s);
 }
 
-// The square root of a positive normal number (anything else: ok false).
-// EXACT: correctly rounded, and the rounding is checked -- s is RN(sqrt(m)) if
-// |m - s^2| < s ulp(s); m - s^2 is a multiple of ulp(s)^2 below 2^54 of them, so
-// the multiply-add gives it exactly -- with ok false for the rare root too close
-// to a midpoint.  Not EXACT: within an ulp.
-template <bool EXACT>
+// The square root of a positive normal number (anything else: ok false), correctly
+// rounded, and the rounding is checked -- s is RN(sqrt(m)) if |m - s^2| < s ulp(s);
+// m - s^2 is a multiple of ulp(s)^2 below 2^54 of them, so the multiply-add gives it
+// exactly -- with ok false for the rare root too close to a midpoint.
 __device__ __forceinline__ double sqrt64(double x, bool &ok) {
   const unsigned hi = d_hi(x);
   ok = ok && hi - 0x00100000u < 0x7fe00000u;
@@ -91,12 +91,10 @@ __device__ __forceinline__ double sqrt64(double x, bool &ok) {
   const double m = __hiloint2double((int)((hi & 0x000fffffu) | (odd ? 0x3ff00000u : 0x40000000u)), (int)d_lo(x));
   const int k = ((int)(hi >> 20) - (odd ? 1023 : 1024)) >> 1;
   const double s = sqrt_core(m);
-  if constexpr (EXACT) {
-    const double r = __fma_rn(-s, s, m);
-    // s in [1, 2]: s ulp(s) = s 2^-52 (2^-51 for s = 2, which only makes the test stricter)
-    const double t = __hiloint2double((int)(d_hi(s) - (52u << 20)), (int)d_lo(s));
-    ok = ok && d_less(__hiloint2double((int)(d_hi(r) & 0x7fffffffu), (int)d_lo(r)), t);
-  }
+  const double r = __fma_rn(-s, s, m);
+  // s in [1, 2]: s ulp(s) = s 2^-52 (2^-51 for s = 2, which only makes the test stricter)
+  const double t = __hiloint2double((int)(d_hi(s) - (52u << 20)), (int)d_lo(s));
+  ok = ok && d_less(__hiloint2double((int)(d_hi(r) & 0x7fffffffu), (int)d_lo(r)), t);
   return __hiloint2double((int)d_hi(s) + (k << 20), (int)d_lo(s));
 }
 
@@ -153,7 +151,7 @@ __device__ __forceinline__ double god64_ref(double m0, double m1, double m2, con
     if (!three) {
       double t = __fma_rn(2.0, p01, -m00);
       t = __dadd_rn(__dadd_rn(__dsub_rn(t, m11), k.q0), k.q1);
-      u = div64(__dadd_rn(__dadd_rn(m1q0, m0q1), __dmul_rn(k.d01, sqrt64<true>(t, ok))), k.s, k.is, ok);
+      u = div64(__dadd_rn(__dadd_rn(m1q0, m0q1), __dmul_rn(k.d01, sqrt64(t, ok))), k.s, k.is, ok);
       three = d_less(m2, u);
     }
     __syncwarp(lanes);  // one pass over the third term for all (see god64_node)
@@ -170,36 +168,47 @@ __device__ __forceinline__ double god64_ref(double m0, double m1, double m2, con
       r = __dadd_rn(__dadd_rn(__dadd_rn(r, k.q01), k.q02), k.q12);
       double n = __dadd_rn(__dmul_rn(__dmul_rn(m2, k.q0), k.q1), __dmul_rn(m1q0, k.q2));
       n = __dadd_rn(n, __dmul_rn(m0q1, k.q2));
-      n = __dadd_rn(n, __dmul_rn(k.d012, sqrt64<true>(r, ok)));
+      n = __dadd_rn(n, __dmul_rn(k.d012, sqrt64(r, ok)));
       u = div64(n, k.den, k.iden, ok);
     }
   }
   return u;
 }
 
-// god_fast64 on sorted minima, with reciprocals for its divisions and the
-// three-term solution first: the two-term one exceeds m2 exactly where the
-// three-term one does (to rounding, and where they meet they are equal), so a node
-// with three terms needs no other.
+// god_fast64 on sorted minima: the same roundings (its sum and product of the
+// two-term numerator and of the three-term result round once, as its expressions
+// contract), but with the three-term solution v first.  Where v exceeds m2 by more
+// than k.sure units of the last place, the two-term one does too, whatever its
+// rounding, and is spared: in exact arithmetic it is the larger of the two, and with
+// r = the largest spacing over the smallest and u = 2^-53 the error of v is below
+// (63 r^3 + 93 r^2 + 50) u v and that of the two-term solution below 20 r u v (the
+// discriminants are at least the square of the inverse of the largest spacing where v
+// is a solution at all, and where it is not, r <= 1000 keeps v below m2).
 __device__ __forceinline__ double god64_fast(double m0, double m1, double m2, const GodPerm64 &k, bool &ok) {
   double u = __dadd_rn(m0, k.d0);
   if (d_less(m1, u)) {
     const double a = __dsub_rn(m1, m0), aa = __dmul_rn(a, a);
     const unsigned lanes = __activemask();
-    bool two = true;
-    if (d_less(m2, u)) {
+    bool three = false, solved = d_less(m2, u);
+    double v = 0.0;
+    if (solved) {
       const double b = __dsub_rn(m2, m0);
       const double B = __fma_rn(a, k.w1, __dmul_rn(b, k.w2));
       const double C = __fma_rn(aa, k.w1, __fma_rn(__dmul_rn(b, b), k.w2, -1.0));
-      const double D = __fma_rn(B, B, __dmul_rn(-k.wsum, C));
-      if (__double_as_longlong(D) > 0) {
-        const double v = __fma_rn(__dadd_rn(B, sqrt64<false>(D, ok)), k.iwsum, m0);
-        two = !d_less(m2, v);
-        if (!two) u = v;
+      bool real = true;
+      v = __fma_rn(__dadd_rn(B, sqrt64(__fma_rn(B, B, __dmul_rn(-k.wsum, C)), real)), k.iwsum, m0);
+      three = real && __double_as_longlong(v) - __double_as_longlong(m2) > k.sure;
+      solved = real;
+      if (three) u = v;
+    }
+    __syncwarp(lanes);  // one pass over the two-term solution for all (see god64_node)
+    if (!three) {
+      u = __dadd_rn(m0, div64(__fma_rn(a, k.w1, sqrt64(__fma_rn(-aa, k.w01, k.ws), ok)), k.ws, k.iws, ok));
+      if (d_less(m2, u)) {
+        ok = ok && solved;
+        u = v;
       }
     }
-    __syncwarp(lanes);
-    if (two) u = __fma_rn(__fma_rn(a, k.w1, sqrt64<false>(__fma_rn(-aa, k.w01, k.ws), ok)), k.iws, m0);
   }
   return u;
 }

@@ -43,7 +43,8 @@ struct GodPerm64 {
   double ws, iws;        // w0 + w1, 1 / ws
   double wsum, iwsum;    // w of all axes, 1 / wsum
   float r0, r1, rm, rd;  // 1 / d0, 1 / d1, 1 / min(d0, d1), (d0 + d1) / min(d0, d1)
-  double pad;            // rows of 23 doubles: six of them read at once share no bank
+  long long sure;        // god64_fast: v above m2 by more of its last places needs three terms
+                         // (rows of 23 doubles: six of them read at once share no bank)
 };
 
 // Per-sweep constants of the local solver.

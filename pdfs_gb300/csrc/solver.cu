@@ -475,6 +475,7 @@ static void fill_perm(const pdfs_grid &g, GodPerm64 out[6]) {
   const double h[3] = {g.dx, g.dy, g.dz};
   auto mul = [](double a, double b) { volatile double r = a * b; return (double)r; };
   auto add = [](double a, double b) { volatile double r = a + b; return (double)r; };
+  const double r = std::max(g.dx, std::max(g.dy, g.dz)) / std::min(g.dx, std::min(g.dy, g.dz));
   double wsum = 0.0;
   for (int i = 0; i < 3; ++i) wsum = add(wsum, 1.0 / mul(h[i], h[i]));
   for (int a0 = 0; a0 < 3; ++a0)
@@ -507,6 +508,7 @@ static void fill_perm(const pdfs_grid &g, GodPerm64 out[6]) {
       p.r1 = (float)(1.0 / d1);
       p.rm = (float)(1.0 / std::min(d0, d1));
       p.rd = (float)((d0 + d1) / std::min(d0, d1));
+      p.sure = r <= 1000.0 ? (long long)(256.0 * (r * r * r + r * r) + 128.0) : INT64_MAX;
     }
 }
 
@@ -760,8 +762,8 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 //     bricks save in the chain they lose once the chip is full.
 //   reference and fast: bricks of 8 x 8 x 16 with the solvers of god64.cuh.
 //     Reference 0.54 / 3.3 / 8.8 / 3.5 / -, pencils 1.35 / 10.5 / 18.7 / - / -; fast
-//     0.29 / 1.5 / 4.0 / 1.8 / -, pencils 0.82 / 5.6 / 10.4 / - / -.  A level costs one
-//     warp 16 to 61 FP64 operations of 64 cycles each however few of its lanes hold
+//     0.34 / 1.8 / 4.4 / 2.0 / -, pencils 0.82 / 5.6 / 10.4 / - / -.  A level costs one
+//     warp 18 to 61 FP64 operations of 64 cycles each however few of its lanes hold
 //     a node, so small faces, which lag their upwind bricks by fewer levels, win:
 //     16 x 16 x 16 bricks take 5 to 50 % more.
 constexpr long long kPairBrickNodes = 1ll << 26;
