@@ -460,7 +460,7 @@ extern "C" int pdfs_solve_batch(int n, const pdfs_grid *grids, double *const *fi
   };
   for (int g = 0; g < n; ++g) {
     if (!fields[g]) return cleanup(PDFS_ERR_INVALID);
-    if ((rc = pdfs_ctx_create(&grids[g], &o, &ctx[g]))) return cleanup(rc);
+    if ((rc = ctx_create(&grids[g], &o, &ctx[g], true))) return cleanup(rc);
     if ((rc = pdfs_ctx_load(ctx[g], fields[g], frozen ? frozen[g] : nullptr))) return cleanup(rc);
   }
   B.dev = ctx[0]->dev;

@@ -207,6 +207,9 @@ struct Handles {
   cudaStream_t st2 = nullptr;
   cudaEvent_t slab_ev[kSlabs + 1] = {};
 };
+// pdfs_ctx_create; batch: for a batch's rounds, which sweep on columns or pencils (no
+// bricks' mailboxes or orders of plain sweeps).
+int ctx_create(const pdfs_grid *g, const pdfs_opts *o, pdfs_ctx **out, bool batch);
 cudaError_t handles_take(int dev, Handles *h);
 // Device memory from the cache of idle blocks, or new; given back idle.
 cudaError_t block_take(int dev, void **out, size_t bytes);
@@ -248,7 +251,12 @@ struct pdfs_ctx {
     int *tord = nullptr;
   } plain32, plain64;
   int epoch = 0;  // flag value of the last brick or pencil sweep
-  unsigned long long *pmail = nullptr;  // pencils: epoch-tagged face mailboxes
+  // epoch-tagged face mailboxes of bricks and pencils, a block of their own: where
+  // the device has no room for the bricks' they are left out (brick_mail false), and
+  // bricks wait for whole upwind bricks
+  unsigned long long *pmail = nullptr;
+  size_t pmail_bytes = 0, pencil_words = 0;  // pencil_words: 64-bit words the pencils need of it
+  bool brick_mail = false;
   int prow = 0;                          // their diagonals per face
   // lane-column tiles: ticket orders, and the epoch-tagged face mailboxes
   int *lcord32 = nullptr, *lcord64 = nullptr;

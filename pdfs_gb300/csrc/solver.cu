@@ -795,7 +795,33 @@ static void pick_tiles(pdfs_ctx *c) {
   }
 }
 
-extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_ctx **out) {
+// A block of `words` mailbox words, every tag 0 (which never matches: epochs start at 1).
+static cudaError_t take_mail(pdfs_ctx *c, size_t words) {
+  c->pmail = nullptr;
+  c->pmail_bytes = 0;
+  if (!words) return cudaSuccess;
+  void *p = nullptr;
+  cudaError_t e = block_take(c->dev, &p, words * 8);
+  if (e != cudaSuccess) return e;
+  c->pmail = (unsigned long long *)p;
+  c->pmail_bytes = words * 8;
+  return cudaMemsetAsync(c->pmail, 0, c->pmail_bytes, c->st);
+}
+
+// Gives the bricks' mailboxes back (the context is idle): the device is full.
+static cudaError_t drop_brick_mail(pdfs_ctx *c) {
+  cudaError_t e = cudaStreamSynchronize(c->st);
+  if (e != cudaSuccess) return e;
+  block_give(c->dev, c->pmail, c->pmail_bytes);
+  c->brick_mail = false;
+  return take_mail(c, c->pencil_words);
+}
+
+extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o, pdfs_ctx **out) {
+  return ctx_create(g, o, out, false);
+}
+
+int pdfs::ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_ctx **out, bool batch) {
   if (!out) return PDFS_ERR_INVALID;
   *out = nullptr;
   pdfs_opts o;
@@ -899,30 +925,31 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
     size_t prog = 0, mb = 0;
     for (int k = 0; k < 2; ++k) {
       const Layout &L = k ? c->L64 : c->L32;
+      const TileShape ts = k ? s64 : s32;
       const size_t ncol = (size_t)L.ncx * L.ncy;
       prog = std::max(prog, ncol * (size_t)L.ty);
-      mb = std::max(mb, ncol * (size_t)nb * (size_t)(L.tx + L.ty) * (size_t)L.esize);
+      if (!ts.bz && !ts.lc)  // columns
+        mb = std::max(mb, ncol * (size_t)nb * (size_t)(L.tx + L.ty) * (size_t)L.esize);
     }
     c->progress_ints = prog;
     c->mailbox_bytes = mb;
   }
   // pencils: two faces of prow diagonals x 16 entries x 2 words per pencil
-  // (tag 0 never matches: epochs start at 1)
-  size_t pmail_words = 0;
-  if (s32.pencil || s64.pencil) {
-    c->prow = g->nz + 15;
-    pmail_words = (size_t)((g->nx + 15) / 16) * ((g->ny + 15) / 16) * 2 * (size_t)c->prow * 16 * 2;
-  }
+  if (s32.pencil || s64.pencil) c->prow = g->nz + 15;
+  if (batch) c->plain32.b = c->plain64.b = 0;
+  if (batch ? s32.pencil || s64.pencil : s64.pencil && !c->plain64.b && o.precision != PDFS_PREC_FP32)
+    c->pencil_words = (size_t)((g->nx + 15) / 16) * ((g->ny + 15) / 16) * 2 * (size_t)c->prow * 16 * 2;
   // bricks: three faces per brick (T3Geo::MAIL words, two per FP64 value)
+  size_t brick_words = 0;
   auto brick_mail = [&](const int nt[3], int bx, int by, int bz, int words) {
-    pmail_words = std::max(pmail_words, (size_t)nt[0] * nt[1] * nt[2] * (size_t)(bz * by + bz * bx + bx * by) * words);
+    brick_words = std::max(brick_words, (size_t)nt[0] * nt[1] * nt[2] * (size_t)(bz * by + bz * bx + bx * by) * words);
   };
   std::vector<int> bp[2];  // ticket orders of the pencil tiles' plain sweeps
   for (int k = 0; k < 2; ++k) {
     const TileShape ts = k ? s64 : s32;
     const int *nt = k ? c->nt64 : c->nt32;
     pdfs_ctx::Plain &p = k ? c->plain64 : c->plain32;
-    if (o.precision == (k ? PDFS_PREC_FP32 : PDFS_PREC_FP64)) {
+    if (batch || o.precision == (k ? PDFS_PREC_FP32 : PDFS_PREC_FP64)) {
       p.b = 0;
       continue;
     }
@@ -971,7 +998,6 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
   want(&c->tflag, nflags * 4);
   want(&c->tact, nflags);
   want(&c->tsparse, nflags ? (nflags + 1) * 4 : 0);
-  want(&c->pmail, pmail_words * 8);
   want(&c->order32, w32.size() * 4);
   want(&c->order64, w64.size() * 4);
   want(&c->lcord32, lo32.size() * 4);
@@ -990,6 +1016,14 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
     }
   }
   mark("allocation");
+  // the mailboxes; without the bricks' where they do not fit (or a test asks for it)
+  c->brick_mail = brick_words > 0 && !getenv("PDFS_TEST_NO_BRICK_MAIL");
+  e = take_mail(c, c->brick_mail ? std::max(c->pencil_words, brick_words) : c->pencil_words);
+  if (e == cudaErrorMemoryAllocation && c->brick_mail) {
+    cudaGetLastError();
+    e = drop_brick_mail(c);
+  }
+  if (e != cudaSuccess) return fail(e);
   GodPerm64 perm[6];
   fill_perm(*g, perm);
   if ((e = cudaMemcpyAsync(c->kperm, perm, sizeof perm, cudaMemcpyHostToDevice, c->st)) != cudaSuccess) return fail(e);
@@ -1010,7 +1044,6 @@ extern "C" int pdfs_ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_c
     if (p.b && bp[k].empty()) p.tord = k ? c->tord64 : c->tord32;  // the masked sweeps' bricks
   }
   if (nflags && (e = cudaMemsetAsync(c->tflag, 0, nflags * 4, c->st)) != cudaSuccess) return fail(e);
-  if (pmail_words && (e = cudaMemsetAsync(c->pmail, 0, pmail_words * 8, c->st)) != cudaSuccess) return fail(e);
   // lane-column mailboxes: tag 0 never matches (epochs start at 1)
   if (lc_y && (e = cudaMemsetAsync(c->lc_ymail, 0, lc_y * 8, c->st)) != cudaSuccess) return fail(e);
   if (lc_x && (e = cudaMemsetAsync(c->lc_xmail, 0, lc_x * 8, c->st)) != cudaSuccess) return fail(e);
@@ -1053,6 +1086,7 @@ extern "C" void pdfs_ctx_destroy(pdfs_ctx *c) {
   if (c->hd.st2) cudaStreamSynchronize(c->hd.st2);
   if (c->st) cudaStreamSynchronize(c->st);
   block_give(c->dev, c->arena, c->arena_bytes);
+  block_give(c->dev, c->pmail, c->pmail_bytes);
   block_give(c->dev, c->stage, c->stage_bytes);
   handles_give(c->dev, &c->hd);
   cudaGetLastError();
@@ -1069,7 +1103,13 @@ static int ensure_stage(pdfs_ctx *c) {
   block_give(c->dev, c->stage, c->stage_bytes);
   c->stage = nullptr;
   c->stage_bytes = 0;
-  CK(block_take(c->dev, (void **)&c->stage, b));
+  cudaError_t e = block_take(c->dev, (void **)&c->stage, b);
+  if (e == cudaErrorMemoryAllocation && c->brick_mail) {  // the bricks' mailboxes make room
+    cudaGetLastError();
+    CK(drop_brick_mail(c));
+    e = block_take(c->dev, (void **)&c->stage, b);
+  }
+  CK(e);
   c->stage_bytes = b;
   return PDFS_OK;
 }
@@ -1364,18 +1404,19 @@ static int run_sweep(pdfs_ctx *c, int which, int sn, const uint8_t *active, unsi
                                                        : ARITH_FAST;
   int grid = 0;
   CK(cudaEventRecord(c->k0, c->st));
-  if (pencil && pl.b) {
+  if (pencil && pl.b && c->brick_mail) {
     a.epoch = ++c->epoch;  // mailbox words of every earlier sweep carry a smaller tag
     a.torder = pl.tord;
     a.ntx = pl.nt[0];
     a.nty = pl.nt[1];
     a.ntz = pl.nt[2];
     CK(launch_sweep_plain(which, pl.b, pl.bz, arith, iso, a, L, c->sms, c->st, &grid));
-  } else if (pencil) {
+  } else if (pencil && !pl.b) {
     a.epoch = ++c->epoch;  // mailbox words of every earlier sweep carry a smaller tag
     CK(launch_sweep_pencils(which, arith, iso, a, L, c->sms, c->st, &grid));
   } else if (ts.bz > 0) {
-    a.epoch = ++c->epoch;  // the flags of every earlier sweep are below it
+    a.epoch = ++c->epoch;  // the mail and flags of every earlier sweep are below it
+    if (!c->brick_mail) a.pmail = nullptr;
     CK(launch_sweep_bricks(which, ts.ty, ts.bz, arith, iso, a, L, c->sms, c->st, &grid));
   } else {
     CK(launch_sweep(which, tile, arith, iso, a, L, which == 2 ? (const void *)c->in64 : nullptr, c->sms, c->st,
@@ -1808,6 +1849,7 @@ static int octant_round(pdfs_ctx *c, int which, int first, int nsw, unsigned ful
   a.oct_bits = bits;
   a.oct_tbits = c->tact;
   a.maxchg = c->ochg;
+  if (!c->brick_mail) a.pmail = nullptr;
   a.epoch = c->epoch + 1;  // sweep j publishes epoch + j
   c->epoch += kOctMax;
   const int *nt = f32 ? c->nt32 : c->nt64;

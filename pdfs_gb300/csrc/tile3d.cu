@@ -1,9 +1,16 @@
-// tile3d.cu -- instantiations and launcher of the brick sweep kernel (tile3d.cuh).
+// tile3d.cu -- instantiations (with mailboxes) and launchers of the brick sweep kernel
+// (tile3d.cuh).
 #include <algorithm>
 
-#include "tile3d_launch.cuh"
+#include "tile3d_dispatch.cuh"
 
 namespace pdfs {
+
+// (tile3d_flags.cu)
+extern template cudaError_t dispatch_bricks<false>(int, int, int, int, bool, const SweepArgs &, const Layout &, int,
+                                                   cudaStream_t, int *);
+extern template cudaError_t dispatch_octant<false>(int, int, bool, const SweepArgs &, const Layout &, int, cudaStream_t,
+                                                   int *);
 
 std::vector<int> brick_order(int ntx, int nty, int ntz) {
   // a brick waits for one brick a level below in each axis: listing bricks by
@@ -22,32 +29,6 @@ std::vector<int> brick_order(int ntx, int nty, int ntz) {
     for (int y = 0; y < nty; ++y)
       for (int x = 0; x < ntx; ++x) o[start[x + y + z]++] = i++;
   return o;
-}
-
-template <int BY, int BZ>
-static cudaError_t dispatch_t3(int which, int arith, bool iso, const SweepArgs &a, const Layout &L, int sms,
-                               cudaStream_t st, int *g) {
-  if (which == 0)
-    return iso ? launch_t3<float, 16, BY, BZ, MODE_MIN, ARITH_FAST, true, false>(a, L, sms, st, g)
-               : launch_t3<float, 16, BY, BZ, MODE_MIN, ARITH_FAST, false, false>(a, L, sms, st, g);
-  {
-    if (which == 1) {
-      if (arith == ARITH_REF) return launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_REF, false, false>(a, L, sms, st, g);
-      if (arith == ARITH_FAST) return launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_FAST, false, false>(a, L, sms, st, g);
-      if (arith == ARITH_PAIR)
-        return iso ? launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_PAIR, true, false>(a, L, sms, st, g)
-                   : launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_PAIR, false, false>(a, L, sms, st, g);
-      return iso ? launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_MIXED, true, false>(a, L, sms, st, g)
-                 : launch_t3<double, 16, BY, BZ, MODE_MIN, ARITH_MIXED, false, false>(a, L, sms, st, g);
-    }
-    if (arith == ARITH_REF) return launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_REF, false, false>(a, L, sms, st, g);
-    if (arith == ARITH_FAST) return launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_FAST, false, false>(a, L, sms, st, g);
-    if (arith == ARITH_PAIR)
-      return iso ? launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_PAIR, true, false>(a, L, sms, st, g)
-                 : launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_PAIR, false, false>(a, L, sms, st, g);
-    return iso ? launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_MIXED, true, false>(a, L, sms, st, g)
-               : launch_t3<double, 16, BY, BZ, MODE_REPLACE, ARITH_MIXED, false, false>(a, L, sms, st, g);
-  }
 }
 
 // Block-masked sweeps: per brick (global brick id), whether one of its 8^3
@@ -244,11 +225,6 @@ int octant_scratch_ints(int ntx, int nty, int ntz) {
   return 2 * kOctMax * n + 2 * kOctMax + 1 + kOctMax * (WL + 1) + kOctMax * WL;
 }
 
-template <class T, int BZ, int MODE, int ARITH, bool ISO>
-static cudaError_t launch_oct(const SweepArgs &a, const Layout &L, int sms, cudaStream_t st, int *grid_used) {
-  return launch_t3<T, 16, 16, BZ, MODE, ARITH, ISO, true>(a, L, sms, st, grid_used);
-}
-
 cudaError_t launch_octant_round(int which, int arith, bool iso, int nsw, const SweepArgs &a0, const Layout &L,
                                 int *list, int *cnt_off, int sms, cudaStream_t st, int *g) {
   // FP32 min-update rounds on the FP32 masked bricks (16 x 16 x 32), FP64
@@ -256,7 +232,7 @@ cudaError_t launch_octant_round(int which, int arith, bool iso, int nsw, const S
   // rounds on 16^3 bricks, 8 CTAs per SM instead of 4, were measured slower
   // on the 768^3 grid: full round 22.4 -> 25.9 ms, masked 13.8 -> 15.0 ms.)
   const int bz = which == 0 ? 32 : 16;
-  if (!a0.tflag || !a0.pmail || !a0.torder || !a0.oct_bits || !a0.oct_tbits || a0.ntx < 1 || L.ty != 16 || L.tx != 16 ||
+  if (!a0.tflag || !a0.torder || !a0.oct_bits || !a0.oct_tbits || a0.ntx < 1 || L.ty != 16 || L.tx != 16 ||
       L.xo != 0 || which == 1 || (which == 2 && (!a0.bcap64 || !a0.bcap32)) || a0.ntz != (a0.nz + bz - 1) / bz ||
       nsw < 1 || nsw > kOctMax || (long long)a0.ntx * a0.nty * a0.ntz >= (1ll << 27))
     return cudaErrorInvalidValue;
@@ -294,28 +270,13 @@ cudaError_t launch_octant_round(int which, int arith, bool iso, int nsw, const S
   a.nticket = off + nsw;  // the round's ticket count
   a.blk_active = nullptr;
   a.tact = nullptr;
-  if (which == 0)
-    return iso ? launch_oct<float, 32, MODE_MIN, ARITH_FAST, true>(a, L, sms, st, g)
-               : launch_oct<float, 32, MODE_MIN, ARITH_FAST, false>(a, L, sms, st, g);
-  switch (arith) {
-    case ARITH_PAIR:
-      return iso ? launch_oct<double, 16, MODE_REPLACE, ARITH_PAIR, true>(a, L, sms, st, g)
-                 : launch_oct<double, 16, MODE_REPLACE, ARITH_PAIR, false>(a, L, sms, st, g);
-    case ARITH_MIXED:
-      return iso ? launch_oct<double, 16, MODE_REPLACE, ARITH_MIXED, true>(a, L, sms, st, g)
-                 : launch_oct<double, 16, MODE_REPLACE, ARITH_MIXED, false>(a, L, sms, st, g);
-    case ARITH_FAST:
-      return launch_oct<double, 16, MODE_REPLACE, ARITH_FAST, false>(a, L, sms, st, g);
-    case ARITH_REF:
-      return launch_oct<double, 16, MODE_REPLACE, ARITH_REF, false>(a, L, sms, st, g);
-    default:
-      return cudaErrorInvalidValue;
-  }
+  return a.pmail ? dispatch_octant<true>(which, arith, iso, a, L, sms, st, g)
+                 : dispatch_octant<false>(which, arith, iso, a, L, sms, st, g);
 }
 
 cudaError_t launch_sweep_bricks(int which, int by, int bz, int arith, bool iso, const SweepArgs &a0, const Layout &L,
                                 int sms, cudaStream_t st, int *g) {
-  if (!a0.pmail || !a0.torder || a0.ntx < 1 || a0.nty < 1 || a0.ntz < 1 || L.ty != by || L.tx != 16 ||
+  if ((!a0.pmail && !a0.tflag) || !a0.torder || a0.ntx < 1 || a0.nty < 1 || a0.ntz < 1 || L.ty != by || L.tx != 16 ||
       L.xo != 0 || (which == 2 && (!a0.bcap64 || !a0.bcap32)))
     return cudaErrorInvalidValue;
   SweepArgs a = a0;
@@ -335,13 +296,12 @@ cudaError_t launch_sweep_bricks(int which, int by, int bz, int arith, bool iso, 
     a.tact = nullptr;
     a.nticket = nullptr;
   }
-  if (by == 16 && bz == 16) return dispatch_t3<16, 16>(which, arith, iso, a, L, sms, st, g);
-  if (by == 16 && bz == 32) return dispatch_t3<16, 32>(which, arith, iso, a, L, sms, st, g);
-  if (by == 8 && bz == 32) return dispatch_t3<8, 32>(which, arith, iso, a, L, sms, st, g);
-  if (by == 8 && bz == 48 && which == 0)  // FP32 only
-    return iso ? launch_t3<float, 16, 8, 48, MODE_MIN, ARITH_FAST, true, false>(a, L, sms, st, g)
-               : launch_t3<float, 16, 8, 48, MODE_MIN, ARITH_FAST, false, false>(a, L, sms, st, g);
-  return cudaErrorInvalidValue;
+  return a.pmail ? dispatch_bricks<true>(which, by, bz, arith, iso, a, L, sms, st, g)
+                 : dispatch_bricks<false>(which, by, bz, arith, iso, a, L, sms, st, g);
 }
+
+template cudaError_t dispatch_bricks<true>(int, int, int, int, bool, const SweepArgs &, const Layout &, int, cudaStream_t,
+                                           int *);
+template cudaError_t dispatch_octant<true>(int, int, bool, const SweepArgs &, const Layout &, int, cudaStream_t, int *);
 
 }  // namespace pdfs

@@ -51,6 +51,11 @@
 // node go to global memory at the brick's end, a row at a time (a store per
 // node as it is computed touches up to 32 lines a warp).
 //
+// MAIL false (tile3d_flags.cu): a brick waits for its visited upwind bricks to finish
+// the sweep, by flag, and its box's copy brings their new values.  For contexts whose
+// device has no room for mailboxes (3 bytes a node for 64-bit values on 16 x 16 x 16
+// bricks, 5 on 8 x 8 x 16).
+//
 // Every wait is bounded (SweepArgs::wait_cycles): on expiry the kernel
 // records DEV_ERR_TIMEOUT, raises the abort flag, lets its own TMA copy land
 // and returns.
@@ -175,8 +180,9 @@ __device__ __forceinline__ int diag_rank(int lx, int ly) {  // the position of c
 // without a visited block are passed over (no brick waits for them).  In a
 // round, the brick and its six face neighbours have to finish their latest
 // earlier sweep first: lanes 0..6 leave in wait_flag a flag that is not there
-// yet (else -1), for t3_wait once the current brick has published its own.
-template <class G, bool OCT>
+// yet (else -1), for t3_wait once the current brick has published its own.  Without
+// mail lanes 7..9 do so for the visited upwind bricks of this sweep.
+template <class G, bool OCT, bool MAIL>
 __device__ __forceinline__ void t3_next(const SweepArgs &a, int ntile, T3Desc &d, volatile int *s_abort,
                                         int &wait_flag, int &wait_epoch) {
   const int lane = threadIdx.x & 31;
@@ -232,7 +238,7 @@ __device__ __forceinline__ void t3_next(const SweepArgs &a, int ntile, T3Desc &d
       const int i = lane - UX - UY;
       on = lk > 0 && visited(bx0 + i % G::NBX, by0 + i / G::NBX, sz > 0 ? bz0 - 1 : bz0 + G::NZB);
     }
-    const unsigned up = __ballot_sync(0xffffffffu, on);
+    const unsigned up = MAIL ? __ballot_sync(0xffffffffu, on) : 0u;
     if constexpr (OCT) {
       // the round's earlier sweeps, lanes 0..6: the brick, then its neighbours
       if (lane < 7) {
@@ -249,6 +255,21 @@ __device__ __forceinline__ void t3_next(const SweepArgs &a, int ntile, T3Desc &d
         if (need >= 0 && ld_acquire_gpu(a.tflag + n) < a.epoch + need) {
           wait_flag = n;
           wait_epoch = a.epoch + need;
+        }
+      }
+      __syncwarp();
+    }
+    if constexpr (!MAIL) {
+      if (lane >= 7 && lane < 10) {
+        const int n = lane == 7   ? (li > 0 ? tile - sx : -1)
+                      : lane == 8 ? (lj > 0 ? tile - sy * ntx : -1)
+                                  : (lk > 0 ? tile - sz * ntx * nty : -1);
+        const int epoch = OCT ? a.epoch + osw : a.epoch;
+        bool want = n >= 0;
+        if (want && !every) want = OCT ? (__ldg(a.oct_tbits + n) & obit) != 0 : __ldg(a.tact + n) != 0;
+        if (want && ld_acquire_gpu(a.tflag + n) < epoch) {
+          wait_flag = n;
+          wait_epoch = epoch;
         }
       }
       __syncwarp();
@@ -435,7 +456,7 @@ __device__ __forceinline__ void t3_receive(const SweepArgs &a, const T3Desc &d, 
 // k_oct_merge) interleaves the sweeps by wavefront level with every brick
 // after the ones it waits on, so every wait is on a smaller ticket.  The
 // result is the sequential sweeps', bit for bit.
-template <class T, int BX_, int BY_, int BZ, int MODE, int ARITH, bool ISO, bool OCT = false>
+template <class T, int BX_, int BY_, int BZ, int MODE, int ARITH, bool ISO, bool OCT = false, bool MAIL = true>
 __global__ void __launch_bounds__(T3GeoOf<T, BX_, BY_, BZ, ARITH>::NT,
                                   (sizeof(T) == 4 || ARITH == ARITH_PAIR) ? T3GeoOf<T, BX_, BY_, BZ, ARITH>::CTAS : 2)
     t3_sweep_kernel(const __grid_constant__ CUtensorMap tm_u, const __grid_constant__ SweepArgs a) {
@@ -486,7 +507,7 @@ __global__ void __launch_bounds__(T3GeoOf<T, BX_, BY_, BZ, ARITH>::NT,
   if (!OCT && tid < G::NB) s_chg[tid] = 0;
   __syncthreads();
   int wait_flag = -1, wait_epoch = 0;  // helper warp: an earlier sweep's flag to wait for
-  if (!compute) t3_next<G, OCT>(a, ntile, s_desc[0], &s_abort, wait_flag, wait_epoch);
+  if (!compute) t3_next<G, OCT, MAIL>(a, ntile, s_desc[0], &s_abort, wait_flag, wait_epoch);
   __syncthreads();
 
   // my column, brick-local x, y in sweep order, by diagonal
@@ -505,11 +526,11 @@ __global__ void __launch_bounds__(T3GeoOf<T, BX_, BY_, BZ, ARITH>::NT,
     // read 0 (never used).  The barrier before orders this CTA's generic accesses
     // to the box (each thread's proxy fence) before the copy's writes; the global
     // fence orders the flags acquired by this warp before the copy's reads.
-    if constexpr (OCT) {
+    if constexpr (OCT || !MAIL) {
       if (!compute) t3_wait(a, wait_flag, wait_epoch, &s_abort);
     }
     if (tid == G::NC) {
-      if constexpr (OCT) fence_proxy_async_global();
+      if constexpr (OCT || !MAIL) fence_proxy_async_global();
       mbar_arrive_tx(bar, G::BOX_BYTES);
       tma_load_3d(box, &tm_u, bi * BX, y0 - 1, z0 - 1, bar);
     }
@@ -549,9 +570,10 @@ __global__ void __launch_bounds__(T3GeoOf<T, BX_, BY_, BZ, ARITH>::NT,
     frozen = __syncthreads_or(frozen) != 0;
     mbar_try(bar, it & 1);  // complete: each thread's own view of the copy's writes
     const bool poisoned = tile == a.poison_col;  // test hook: the brick hands nothing over
+    const bool mute = !MAIL || poisoned;
     if (!compute) {
       t3_receive<T, G>(a, d, tile, d.epoch, box, x0, y0, zcnt, grp, &s_abort);
-      t3_next<G, OCT>(a, ntile, s_desc[(it + 1) & 1], &s_abort, wait_flag, wait_epoch);
+      t3_next<G, OCT, MAIL>(a, ntile, s_desc[(it + 1) & 1], &s_abort, wait_flag, wait_epoch);
     } else {
       // the planes of my column that update, one bit each in sweep order (inside
       // the grid, in a visited block, not frozen).  Read once per brick, off the
@@ -577,12 +599,12 @@ __global__ void __launch_bounds__(T3GeoOf<T, BX_, BY_, BZ, ARITH>::NT,
       // face inside the grid: a reader takes those of visited blocks)
       const bool mx = lx == BX - 1 && d.li < a.ntx - 1, my = ly == BY - 1 && d.lj < a.nty - 1;
       PlaneBits face = 0;
-      if (vxy && !poisoned && (mx || my)) {
+      if (vxy && !mute && (mx || my)) {
         face = zcnt < BZ ? (PlaneBits(1) << zcnt) - 1 : PlaneBits(~0ull >> (64 - BZ));
         if (szd < 0) face = G::flip(face);
       }
       // my z face node, the column's last: its level, where a brick is downwind
-      const int zlev = vxy && !poisoned && d.lk < a.ntz - 1 ? lxy + BZ - 1 : -G::GL;
+      const int zlev = vxy && !mute && d.lk < a.ntz - 1 ? lxy + BZ - 1 : -G::GL;
       // mailbox entry of my face node of level L: row L - foff (the reader's level, wrapped)
       const int foff = mx ? BX - 1 : BY - 1, fcol = mx ? G::MX + ly : G::MY + lx;
       // the levels: node (lx, ly, lz = L - lx - ly), sweep order; live, face and
@@ -730,12 +752,13 @@ __global__ void __launch_bounds__(T3GeoOf<T, BX_, BY_, BZ, ARITH>::NT,
     }
     fence_proxy_async();  // my accesses to the box come before the next copy's writes
     if (__syncthreads_or(s_abort)) break;
-    // the brick is done: publish (a round's later sweeps, if any, wait for it).  The
-    // barrier orders every thread's stores before this thread's GPU-scope fence,
-    // which orders them before the flag.
-    if constexpr (OCT) {
+    // the brick is done: publish (a round's later sweeps, if any, wait for it, and
+    // without mail the downwind bricks).  The barrier orders every thread's stores
+    // before this thread's GPU-scope fence, which orders them before the flag.
+    if constexpr (OCT || !MAIL) {
       if (tid == G::NC && !poisoned && a.tflag) publish_gpu(a.tflag + tile, d.epoch);
-    } else if (a.blk_chg != nullptr && tid < G::NB) {
+    }
+    if (!OCT && a.blk_chg != nullptr && tid < G::NB) {
       // block changes: only nodes inside the grid change, so a positive one names a block of the grid
       if (s_chg[tid]) {
         const int bx = G::NBX * bi + tid % G::NBX, by = G::NBY * bj + (tid / G::NBX) % G::NBY;
