@@ -790,7 +790,7 @@ static void pick_tiles(pdfs_ctx *c) {
   if (tile64(c->t64).pencil) {
     if (c->o.arith == PDFS_ARITH_REFERENCE || c->o.arith == PDFS_ARITH_FAST)
       set(c->plain64, 8, 16);
-    else if (nodes <= kPairBrickNodes)
+    else if (nodes <= kPairBrickNodes && !getenv("PDFS_TEST_PLAIN_PENCILS"))  // (a test asks for pencils)
       set(c->plain64, 16, 32);
   }
 }
