@@ -110,8 +110,8 @@ constexpr int kOctWords = kOctMax + 8;
 int octant_scratch_ints(int ntx, int nty, int ntz);
 cudaError_t launch_octant_round(int which, int arith, bool iso, int nsw, const SweepArgs &a0, const Layout &L,
                                 int *list, int *cnt_off, int sms, cudaStream_t st, int *grid_used);
-// Ticket order of bricks: local brick ids (lk * nty + lj) * ntx + li by level li + lj + lk.
-std::vector<int> brick_order(int ntx, int nty, int ntz);
+// Ticket order of bricks: local brick ids (lk * nty + lj) * ntx + li by level li + lj + wz lk.
+std::vector<int> brick_order(int ntx, int nty, int ntz, int wz = 1);
 cudaError_t encode_field_map(CUtensorMap *m, void *base, int esize, const Layout &L, int nplanes, int bx, int by,
                              int bz);
 

@@ -766,8 +766,22 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 //     warp 18 to 61 FP64 operations of 64 cycles each however few of its lanes hold
 //     a node, so small faces, which lag their upwind bricks by fewer levels, win:
 //     16 x 16 x 16 bricks take 5 to 50 % more.
+//
+// Tickets of the plain bricks, where these have more than kLevelOrderColumns columns,
+// follow the node levels at which bricks can start (a brick of 8 x 8 x 32 begins 8 levels after
+// its x and y neighbours and 32 after its z neighbour).  Listed by the brick levels li +
+// lj + lk instead, the bricks far along z are taken long before they can start, and on a
+// wide grid they fill the chip while others wait for a CTA: 2000 x 4 x 2000 takes 1.97
+// ms FP32, 15.8 reference, 2.92 pairs, with node levels 1.60, 13.5 and 2.61 (pencils: 1.99,
+// 15.1, 2.64); 251 x 233 x 241 reference 3.30 and 3.12.  With fewer bricks most of them
+// are resident in either order, and brick levels spread the running ones better:
+// reference 151 x 127 x 110 (2128 bricks of 64 columns) 1.36 and 1.50, 500 x 4 x 500
+// (2016) 2.95 and 3.35, 700 x 4 x 700 (3872) 4.28 and 4.58; 192 x 176 x 160 (5280) even,
+// 1000 x 4 x 1000 (7875) 6.69 and 6.45; pairs, 256 columns a brick, 500 x 8 x 500 (512)
+// 0.604 and 0.611, 1000 x 4 x 1000 (2016) 1.25 and 1.24.
 constexpr long long kPairBrickNodes = 1ll << 26;
 constexpr long long kSmallBrickLevel = 30000;
+constexpr long long kLevelOrderColumns = 7000 * 64;
 
 static void pick_tiles(pdfs_ctx *c) {
   const int t32 = c->o.tile & 0xff, t64 = (c->o.tile >> 8) & 0xff;
@@ -956,7 +970,9 @@ int pdfs::ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_ctx **out, 
     if (ts.bz) brick_mail(nt, ts.tx, ts.ty, ts.bz, k ? 2 : 1);
     if (!p.b) continue;
     brick_mail(p.nt, p.b, p.b, p.bz, k ? 2 : 1);
-    if (p.b != ts.tx || p.bz != ts.bz) bp[k] = brick_order(p.nt[0], p.nt[1], p.nt[2]);
+    if (p.b != ts.tx || p.bz != ts.bz)
+      bp[k] = brick_order(p.nt[0], p.nt[1], p.nt[2],
+                          (long long)p.nt[0] * p.nt[1] * p.nt[2] * p.b * p.b > kLevelOrderColumns ? p.bz / p.b : 1);
   }
   std::vector<std::pair<void **, size_t>> plan;
   auto want = [&](auto **p, size_t bytes) {

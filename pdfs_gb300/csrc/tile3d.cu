@@ -12,22 +12,22 @@ extern template cudaError_t dispatch_bricks<false>(int, int, int, int, bool, con
 extern template cudaError_t dispatch_octant<false>(int, int, bool, const SweepArgs &, const Layout &, int, cudaStream_t,
                                                    int *);
 
-std::vector<int> brick_order(int ntx, int nty, int ntz) {
-  // a brick waits for one brick a level below in each axis: listing bricks by
-  // level (x + y + z), in index order within a level, lists all three first,
+std::vector<int> brick_order(int ntx, int nty, int ntz, int wz) {
+  // a brick waits for one brick below it in each axis: listing bricks by level
+  // (x + y + wz z, wz >= 1), in index order within a level, lists all three first,
   // which is all the deadlock argument needs.  A counting sort by level.
   const size_t n = (size_t)ntx * nty * ntz;
-  const int levels = ntx + nty + ntz - 2;
+  const int levels = ntx + nty + wz * (ntz - 1) - 1;
   std::vector<size_t> start((size_t)levels + 1, 0);
   for (int z = 0; z < ntz; ++z)
     for (int y = 0; y < nty; ++y)
-      for (int x = 0; x < ntx; ++x) ++start[x + y + z + 1];
+      for (int x = 0; x < ntx; ++x) ++start[x + y + wz * z + 1];
   for (int l = 0; l < levels; ++l) start[l + 1] += start[l];
   std::vector<int> o(n);
   int i = 0;
   for (int z = 0; z < ntz; ++z)
     for (int y = 0; y < nty; ++y)
-      for (int x = 0; x < ntx; ++x) o[start[x + y + z]++] = i++;
+      for (int x = 0; x < ntx; ++x) o[start[x + y + wz * z]++] = i++;
   return o;
 }
 

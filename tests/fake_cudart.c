@@ -4,6 +4,8 @@
  * frees, enqueues or waits, one line each, to the file FAKE_LOG names.
  *   FAKE_MEMORY  bytes of the device: an allocation past them fails
  *   FAKE_FAIL    part of a kernel's name: its first launch returns an error
+ *   FAKE_COPIES, FAKE_COPY_BYTES  a file to append the host data of copies of so many
+ *                bytes to
  * Device-to-host copies leave their target as it is (pinned memory starts at zero: no
  * error, no change), so a solve ends after its first sweeps. */
 #define _GNU_SOURCE
@@ -142,7 +144,13 @@ int cudaMemcpy(void *d, const void *s, size_t n, int k) {
   return 0;
 }
 int cudaMemcpyAsync(void *d, const void *s, size_t n, int k, void *st) {
-  (void)d; (void)s; (void)k;
+  (void)d; (void)k;
+  const char *f = getenv("FAKE_COPIES"), *b = getenv("FAKE_COPY_BYTES");
+  if (f && b && (size_t)atoll(b) == n && (uint64_t)(uintptr_t)s < BASE) {
+    FILE *o = fopen(f, "ab");
+    fwrite(s, 1, n, o);
+    fclose(o);
+  }
   SAY("copy %zu stream%d\n", n, (int)(intptr_t)st);
   return 0;
 }

@@ -35,3 +35,12 @@ def run(code, memory=None, fail=None, env=None):
         r = subprocess.run([sys.executable, "-c", pre + code], env=e, cwd=ROOT, text=True, capture_output=True)
         assert r.returncode == 0, r.stderr[-2000:]
         return r.stdout, [line.split() for line in open(log)]
+
+
+def copies(code, nbytes):
+    """The host data of every copy to the device of nbytes bytes, in order."""
+    with tempfile.TemporaryDirectory() as d:
+        f = os.path.join(d, "copies")
+        run(code, env={"FAKE_COPIES": f, "FAKE_COPY_BYTES": str(nbytes)})
+        data = open(f, "rb").read() if os.path.exists(f) else b""
+    return [data[i:i + nbytes] for i in range(0, len(data), nbytes)]
