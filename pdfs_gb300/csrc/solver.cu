@@ -766,6 +766,12 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 //     warp 18 to 61 FP64 operations of 64 cycles each however few of its lanes hold
 //     a node, so small faces, which lag their upwind bricks by fewer levels, win:
 //     16 x 16 x 16 bricks take 5 to 50 % more.
+// Mixed sweeps run on pencils where the grid is long in z and thin in y, with levels
+// wide enough to fill some bricks but pencils few enough to run side by side: bricks
+// leave threads idle there, and what is left of their chain is not worth it (bricks /
+// pencils 3.68 / 3.27 on 2000 x 4 x 2000, 1.76 / 1.64 on 1000 x 4 x 1000, 4.33 / 3.76 on
+// 2000 x 12 x 2000, 2.28 / 2.10 on 1000 x 24 x 1000; past the line 0.60 / 0.63 on 300 x
+// 16 x 300, 3.13 / 3.65 on 1400 x 24 x 1400, 5.67 / 7.62 on 4 x 3000 x 3000).
 //
 // Tickets of the plain bricks, where these have more than kLevelOrderColumns columns,
 // follow the node levels at which bricks can start (a brick of 8 x 8 x 32 begins 8 levels after
@@ -782,6 +788,13 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 constexpr long long kPairBrickNodes = 1ll << 26;
 constexpr long long kSmallBrickLevel = 30000;
 constexpr long long kLevelOrderColumns = 7000 * 64;
+
+// Mixed arithmetic on pencils (the comment above).
+static bool mixed_pencils(const pdfs_grid &g) {
+  const long long nodes = (long long)g.nx * g.ny * g.nz, pencils = (long long)((g.nx + 15) / 16) * ((g.ny + 15) / 16);
+  return g.ny >= 2 && g.nz >= 25ll * g.ny && nodes >= 900ll * ((long long)g.nx + g.ny + g.nz) &&
+         (pencils <= 152 || (g.ny <= 12 && g.nz >= g.nx));
+}
 
 static void pick_tiles(pdfs_ctx *c) {
   const int t32 = c->o.tile & 0xff, t64 = (c->o.tile >> 8) & 0xff;
@@ -804,7 +817,8 @@ static void pick_tiles(pdfs_ctx *c) {
   if (tile64(c->t64).pencil) {
     if (c->o.arith == PDFS_ARITH_REFERENCE || c->o.arith == PDFS_ARITH_FAST)
       set(c->plain64, 8, 16);
-    else if (nodes <= kPairBrickNodes && !getenv("PDFS_TEST_PLAIN_PENCILS"))  // (a test asks for pencils)
+    else if (nodes <= kPairBrickNodes && !(c->o.arith == PDFS_ARITH_MIXED && mixed_pencils(c->g)) &&
+             !getenv("PDFS_TEST_PLAIN_PENCILS"))  // (a test asks for pencils)
       set(c->plain64, 16, 32);
   }
 }

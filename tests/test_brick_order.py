@@ -47,3 +47,19 @@ def test_order(shape, kw, b, bz, wz):
     for d, m in ((1, i), (nt[0], j), (nt[0] * nt[1], k)):
         up = m > 0
         assert (at[o[up] - d] < np.arange(n)[up]).all()
+
+
+@pytest.mark.parametrize("shape,pencils", [((1000, 4, 1000), True), ((2000, 12, 2000), True), ((1000, 24, 1000), True),
+                                           ((200, 8, 1000), True), ((1000, 1, 1000), False), ((300, 16, 300), False),
+                                           ((1400, 24, 1400), False), ((4, 1000, 1000), False), ((64, 64, 64), False)])
+def test_mixed_sweeps_of_thin_grids(shape, pencils):
+    code = """
+with api.Context(*%r, (1.0, 1.0, 1.0), precision=L.PREC_FP64, arith=L.ARITH_%s, max_sweeps=8) as c:
+    c.load(np.zeros(tuple(n + 2 for n in %r)))
+    c.run()
+"""
+    for arith, want in (("MIXED", pencils), ("PAIR", False)):
+        _, log = fakecuda.run(code % (shape, arith, shape[::-1]))
+        names = [w[1] for w in log if w[0] == "launch"]
+        assert any("pc_sweep_kernel" in n for n in names) == want
+        assert any("t3_sweep_kernel" in n for n in names) == (not want)
