@@ -208,7 +208,7 @@ def kernel_name(kind, tile, prec, arith):
     k = kernel_kind(kind, tile)
     if k == "brick":
         by, bz = (BRICKS32 if kind == "fp32" else BRICKS64)[tid]
-        return "t3_sweep_kernel<%s, %d, %d, %s, %s>" % (t, by, bz, mode, ar)
+        return "t3_sweep_kernel<%s, 16, %d, %d, %s, %s>" % (t, by, bz, mode, ar)
     if k == "pencil":
         return "pc_sweep_kernel<%s, %s, %s>" % (t, mode, ar)
     if k == "lanecol":
@@ -218,19 +218,47 @@ def kernel_name(kind, tile, prec, arith):
     return "ws_sweep_kernel<%s, %d, %d, %s, %s>" % ((t,) + ty + (mode, ar))
 
 
-def traffic_per_launch(kind, prec, nodes, tile, masked=False, full_round=False):
+def plain_kernel(kind, tile, prec, arith, nx, ny, nz):
+    """The kernel that runs a grid's plain sweeps: the tile's own, but for the pencil
+    tiles, whose plain sweeps run bricks wherever these are faster (pick_tiles in
+    pdfs_gb300/csrc/solver.cu)."""
+    from pdfs_gb300 import _lib as L
+    name = kernel_name(kind, tile, prec, arith)
+    if kernel_kind(kind, tile) != "pencil":
+        return name
+    nodes, span = nx * ny * nz, nx + ny + nz
+    if kind == "fp32":
+        b = (8, 8, 32) if nodes <= 30000 * span else (16, 16, 32)
+    elif arith in (L.ARITH_REFERENCE, L.ARITH_FAST):
+        b = (8, 8, 16)
+    else:
+        pencils = -(-nx // 16) * -(-ny // 16)
+        thin = arith == L.ARITH_MIXED and ny >= 2 and nz >= 25 * ny and nodes >= 900 * span and \
+            (pencils <= 152 or (ny <= 12 and nz >= nx))
+        if nodes > 1 << 26 or thin:
+            return name
+        b = (16, 16, 32)
+    t, rest = name.split("<")[1].split(", ", 1)
+    return "t3_sweep_kernel<%s, %d, %d, %d, %s" % ((t,) + b + (rest,))
+
+
+def traffic_per_launch(kind, prec, nodes, tile, masked=False, full_round=False, kernel=None):
     """DRAM bytes of one launch of the dominant sweep kernel: the per-update
     traffic an ncu capture measured (profiles/traffic.json, dram__bytes_read
     + dram__bytes_write over the capture's executed voxel updates) times this
     launch's updates; None without a capture for that kernel.  masked: the
     block-masked sweeps (bricks), whose traffic per executed update differs
-    from a full sweep's; full_round: the FP32 first cycle as one unmasked round."""
+    from a full sweep's; full_round: the FP32 first cycle as one unmasked round;
+    kernel: the full sweeps' kernel where it is not the tile's own (plain_kernel)."""
     from pdfs_gb300 import _lib as L
     try:
         t = json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))
     except (OSError, ValueError):
         return None
     key = "fp32" if kind == "fp32" else ("fp64_replace" if prec == L.PREC_FP32_POLISH64 else "fp64_min")
+    if kernel and not masked and not full_round and kernel_kind(kind, tile) == "pencil" and kernel.startswith("t3_"):
+        e = next((v for k, v in t.items() if v["kernel"].startswith(kernel[:-1]) and k.endswith("_plain_brick")), None)
+        return None if not e else float(e["dram_bytes_per_update"]) * nodes
     key += "_masked_brick" if masked else ("_round" if full_round else "_" + kernel_kind(kind, tile))
     e = t.get(key)
     return None if not e else float(e["dram_bytes_per_update"]) * nodes
@@ -621,12 +649,12 @@ def main():
                           "launches": max(1, nmask // 8) if rounds else nmask, "updates": umask,
                           "bytes_per_update": per, "one_launch_per_8_sweeps": rounds})
     for q in parts:
-        q["kernel"] = kernel_name(q["phase"], st["tile"], prec, arith) if q["kind"] == "full" else \
-            ("t3_sweep_kernel<float, 16, 32, MIN, FAST>" if q["phase"] == "fp32" else
-             f"t3_sweep_kernel<double, 16, 16, {'REPLACE' if prec == L.PREC_FP32_POLISH64 else 'MIN'}, "
+        q["kernel"] = plain_kernel(q["phase"], st["tile"], prec, arith, w.nx, w.ny, w.nz) if q["kind"] == "full" else \
+            ("t3_sweep_kernel<float, 16, 16, 32, MIN, FAST>" if q["phase"] == "fp32" else
+             f"t3_sweep_kernel<double, 16, 16, 16, {'REPLACE' if prec == L.PREC_FP32_POLISH64 else 'MIN'}, "
              f"{ {L.ARITH_PAIR: 'PAIR', L.ARITH_MIXED: 'MIXED', L.ARITH_FAST: 'FAST'}.get(arith, 'REF')}>")
         if q.get("full_round"):
-            q["kernel"] = "t3_sweep_kernel<float, 16, 32, MIN, FAST, octant round (every block)>"
+            q["kernel"] = "t3_sweep_kernel<float, 16, 16, 32, MIN, FAST, octant round (every block)>"
         if q.get("one_launch_per_8_sweeps"):
             q["kernel"] = q["kernel"][:-1] + ", octant round>"
         q["ms_per_launch"] = q["ms"] / q["launches"]
@@ -638,7 +666,8 @@ def main():
     if dom is not None:
         # traffic: ncu DRAM bytes per update of this kernel (profiles/traffic.json) x its updates per launch
         tr = traffic_per_launch(dom["phase"], prec, dom["updates"] / dom["launches"], st["tile"],
-                                masked=dom["kind"] == "masked", full_round=bool(dom.get("full_round")))
+                                masked=dom["kind"] == "masked", full_round=bool(dom.get("full_round")),
+                                kernel=dom["kernel"])
         roof = {"bound": "hbm", "achieved": dom["achieved_gbs"], "peak": hbm, "unit": "GB/s", "frac": dom["frac"],
                 "traffic": tr, "kernel": dom["kernel"],
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (burst copy)" if "hbm_gbs" in pk else "fallback 6800 GB/s",
