@@ -141,10 +141,15 @@ __device__ __forceinline__ double god_fast64(double m0, double m1, double m2, co
 }
 
 // sqrt of a discriminant of god32s.  FTZ: the flushing approximate root, which
-// has the same bits as the plain one on normal arguments and needs no scaling
-// steps around it (3 % of the 768^3 octant rounds).  A discriminant is 0 or at
-// least about 1e-8 h^2, so only spacings near the ends of the float range
-// (GodConst32::tiny) make a subnormal one: they take FTZ = false.
+// gives the plain one's bits on normal arguments (tests/test_gpu_brick_mail.py
+// compares them) and takes 3 % off the 768^3 octant rounds.  The candidate that is
+// selected has no subnormal discriminant unless the spacings are extreme (one that is
+// not selected may have any).  The two-term one is taken for a < h0 only: 2 h^2 - a^2 >
+// h^2, or q0 + q1 - a^2 q0 q1 > q0.  The three-term one is taken where its value exceeds
+// every minimum: with y_i >= 0 its distances from them, the sum of q_i y_i^2 is 1 and
+// the discriminant the square of the sum of q_i y_i, at least the smallest q (isotropic,
+// times h^4: h^2).  With spacings of 1e-14 to 1e14 (else GodConst32::tiny, and FTZ =
+// false) that is 1e-28 or more.
 template <bool FTZ>
 __device__ __forceinline__ float sqrt_disc(float x) {
   if constexpr (FTZ) {
@@ -189,7 +194,7 @@ __device__ __forceinline__ float god32s(float m0, float m1, float m2, const GodC
     const float sq = q0 + q1;
     const float n2 = fmaf(a, q1, sqrt_disc<FTZ>(fmaxf(fmaf(-a * a, q0 * q1, sq), 0.0f)));
     float u2;
-    if constexpr (FTZ) {  // m0 + n2 / sq as the plain form compiles: a reciprocal and one multiply-add
+    if constexpr (FTZ) {  // m0 + n2 / sq by an approximate reciprocal and one multiply-add: the plain form's bits (tested)
       float rs;
       asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(sq));
       u2 = __fmaf_rn(n2, rs, m0);

@@ -1,5 +1,5 @@
 // pencil.cu -- instantiations and launcher of the pencil sweep kernel (pencil.cuh):
-// the FP32-pair and mixed sweeps of large grids.  Every other plain sweep of the
+// the FP32-pair and mixed sweeps of large grids, and mixed ones of thin grids.  Every other plain sweep of the
 // pencil tiles runs on bricks (tile3d_plain.cu).
 #include <algorithm>
 

@@ -30,7 +30,8 @@
 //     always running or done; every wait is bounded (SweepArgs::wait_cycles)
 //     and ends in DEV_ERR_TIMEOUT plus the abort flag, never in a hang.
 // Sweeps with a block mask or block-change output run on bricks instead, and so do
-// the plain ones but for pairs and mixed on large grids and batches (pick_tiles).
+// the plain ones but for pairs and mixed on large grids, mixed on thin ones, and
+// batches (pick_tiles).
 #pragma once
 #include "sweep.cuh"
 
@@ -105,7 +106,7 @@ __device__ __forceinline__ const SweepArgs &pc_args(const SweepArgs &a0) {
 // sweep s before any grid's sweep s + 1, so every wait is on smaller tickets.  A
 // round is bound by the chain of its largest grids' 8 sweeps: waiting for a grid's
 // whole sweep s - 1 instead made that chain 8 full sweeps long (32 grids of 32 to
-// 160 nodes a side: 17.3 ms, this 16.3; 12 of 24 to 154: 6.4 and 4.9; 7 of 24 to 171:
+// 160 nodes a side: 15.7 ms, this 15.2; 12 of 24 to 154: 6.4 and 4.9; 7 of 24 to 171:
 // 4.9 and 3.6).
 template <class T, int MODE, int ARITH, bool ISO, bool BATCH = false>
 __global__ void __launch_bounds__(PcGeo<T>::NT) pc_sweep_kernel(const __grid_constant__ CUtensorMap tm_u,

@@ -618,7 +618,7 @@ void pdfs::block_give(int dev, void *p, size_t bytes) {
 // Idle sets of handles, at most kMostHandles a process (a batch of 32 grids takes
 // 33): given back with the block cache.  A 37 x 22 x 19 sweep through the one-call
 // API took 707 us making and destroying its own, 373 with the pool;
-// a batch of 32 grids to 160^3 16.4 and 15.5 ms.
+// a batch of 32 grids to 160^3 16.0 and 15.1 ms.
 namespace {
 constexpr size_t kMostHandles = 64;
 struct HandlePool {
@@ -748,17 +748,20 @@ static int validate(const pdfs_grid *g, const pdfs_opts *o) {
 // Plain sweeps of the pencil tiles (no mask, no block changes), ms a sweep on
 // 64^3 / 251 x 233 x 241 / 384^3 / 1000 x 60 x 50 / 768^3 nodes:
 //   FP32: bricks of 8 x 8 x 32 while a level of the sweep holds at most 30000 nodes on
-//     average, 0.074 / 0.34 / (0.75) / 0.47 / (4.1), else of 16 x 16 x 32, (0.079) /
-//     (0.37) / 0.68 / (0.51) / 3.15; pencils take 0.120 / 0.52 / 1.04 / 0.71 / 3.94.
+//     average, 0.073 / 0.34 / (0.71) / 0.48 / (4.2), else of 16 x 16 x 32, (0.077) /
+//     (0.39) / 0.70 / (0.53) / 3.27; pencils took 0.120 / 0.52 / 1.04 / 0.71 / 3.94.
 //     Small faces shorten the chain (8 levels a brick crossed instead of 16), but
 //     their halos are read and their faces mailed twice as often, which is what counts
-//     once the levels fill the chip: both are even at 288^3 (27600 nodes a level: 0.444
-//     and 0.451), 322^3 (34600) takes 0.57 and 0.54, 512 x 512 x 128 (29100) 0.64 and 0.73.
+//     once the levels fill the chip.  On both sides of the line: 288^3 (27600 nodes a
+//     level) 0.43 and 0.47, 512 x 512 x 128 (29100) 0.58 and 0.66, 322^3 (34600) 0.53
+//     and 0.55, 360^3 (43200) 0.64 and 0.64, 384^3 (49200) 0.71 and 0.70.  (The line was
+//     drawn when tickets followed the brick levels, where both were even at 288^3.)
 //   pairs and mixed: bricks of 16 x 16 x 32 up to 2^26 nodes, pencils above.  Pairs
-//     0.117 / 0.53 / 1.11 / 0.75 / 7.3, pencils 0.164 / 0.70 / 1.25 / 0.96 / 5.6; mixed
-//     0.175 / 0.83 / 1.71 / - / 9.8 and 0.214 / 1.00 / 1.79 / - / 8.5; both are even at
-//     448^3 (9.0e7 nodes: 1.57 and 1.63, 2.38 and 2.39).  A box of 64-bit values
-//     leaves room for two CTAs, and a brick reads its halo (27 % more bytes): what
+//     0.117 / 0.54 / 1.14 / 0.80 / 7.7, pencils 0.162 / 0.71 / 1.25 / 1.01 / 5.8; mixed
+//     0.173 / 0.84 / 1.72 / 1.23 / 10.0 and 0.211 / 1.01 / 1.80 / 1.42 / 8.7.  Near the
+//     line: 400^3 (6.4e7 nodes) 1.26 and 1.34, 1.88 and 1.91; 420^3 (7.4e7) 1.45 and
+//     1.49, 2.16 and 2.16; 500^3 (1.25e8) 2.21 and 2.12, 3.22 and 3.11.  A box of 64-bit
+//     values leaves room for two CTAs, and a brick reads its halo (27 % more bytes): what
 //     bricks save in the chain they lose once the chip is full.
 //   reference and fast: bricks of 8 x 8 x 16 with the solvers of god64.cuh.
 //     Reference 0.54 / 3.3 / 8.8 / 3.5 / -, pencils 1.35 / 10.5 / 18.7 / - / -; fast
