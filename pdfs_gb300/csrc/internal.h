@@ -196,10 +196,15 @@ namespace pdfs {
 // The CUDA objects a solve needs beside device memory.  Making and destroying a
 // set costs some 0.1 ms (the pinned block most of it), so idle sets are pooled
 // (solver.cu): a taken set belongs to its taker alone until it is given back,
-// with its streams idle.
+// with its streams idle.  Sets and blocks belong to the CUDA context that they were
+// made in (a cudaDeviceReset ends it, and with it all that it held): the pools know it
+// by its id, and drop what an ended one left.
 constexpr int kSlabs = 32;
 constexpr size_t kPinned = 16384;
+// Id of the calling thread's current driver context, 0 if it cannot be told (noalloc.cu).
+unsigned long long current_ctx_id();
 struct Handles {
+  unsigned long long ctx = 0;  // the context that they were made in
   cudaStream_t st = nullptr;
   cudaEvent_t ev[8] = {};
   char *pinned = nullptr;  // kPinned bytes

@@ -67,7 +67,7 @@ F driver_fn(const char *name, int version) {
   return nullptr;
 }
 
-// Id of the calling thread's current driver context, 0 if it cannot be told.
+}  // namespace
 unsigned long long current_ctx_id() {
   static const CtxGetCurrentFn get_cur = driver_fn<CtxGetCurrentFn>("cuCtxGetCurrent", 4000);
   static const CtxGetIdFn get_id = driver_fn<CtxGetIdFn>("cuCtxGetId", 12000);
@@ -76,6 +76,7 @@ unsigned long long current_ctx_id() {
   if (!get_cur || !get_id || get_cur(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS) return 0;
   return id;
 }
+namespace {
 
 // g_scratch's device address in the current context of device dev.  The
 // lookup runs once per context (cudaGetSymbolAddress also makes the device's

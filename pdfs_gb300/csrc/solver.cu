@@ -523,6 +523,7 @@ static void fill_perm(const pdfs_grid &g, GodPerm64 out[6]) {
 namespace {
 struct CachedBlock {
   int dev;
+  unsigned long long ctx;
   void *p;
   size_t bytes;
 };
@@ -548,21 +549,27 @@ size_t cache_cap(int dev) {
   }
   return cap[dev];
 }
+// Takes a device's blocks out of the cache (the cache locked): into drop those of
+// context ctx, and, unless all is set, only those of other contexts, whose memory is gone.
+void cache_clear(BlockCache &bc, int dev, unsigned long long ctx, bool all, std::vector<void *> *drop) {
+  for (size_t i = 0; i < bc.blocks.size();) {
+    const CachedBlock b = bc.blocks[i];
+    if (b.dev == dev && (all || b.ctx != ctx)) {
+      if (b.ctx == ctx) drop->push_back(b.p);
+      bc.held[dev] -= b.bytes;
+      bc.blocks[i] = bc.blocks.back();
+      bc.blocks.pop_back();
+    } else {
+      ++i;
+    }
+  }
+}
 void cache_release(int dev) {
   std::vector<void *> drop;
   {
     BlockCache &bc = block_cache();
     std::lock_guard<std::mutex> lk(bc.m);
-    for (size_t i = 0; i < bc.blocks.size();) {
-      if (bc.blocks[i].dev == dev) {
-        drop.push_back(bc.blocks[i].p);
-        bc.held[dev] -= bc.blocks[i].bytes;
-        bc.blocks[i] = bc.blocks.back();
-        bc.blocks.pop_back();
-      } else {
-        ++i;
-      }
-    }
+    cache_clear(bc, dev, current_ctx_id(), true, &drop);
   }
   for (void *p : drop) cudaFree(p);
 }
@@ -573,6 +580,7 @@ cudaError_t pdfs::block_take(int dev, void **out, size_t bytes) {
   if (dev >= 0 && dev < 64) {
     BlockCache &bc = block_cache();
     std::lock_guard<std::mutex> lk(bc.m);
+    cache_clear(bc, dev, current_ctx_id(), false, nullptr);
     int best = -1;
     for (size_t i = 0; i < bc.blocks.size(); ++i) {
       const CachedBlock &b = bc.blocks[i];
@@ -607,7 +615,7 @@ void pdfs::block_give(int dev, void *p, size_t bytes) {
     BlockCache &bc = block_cache();
     std::lock_guard<std::mutex> lk(bc.m);
     if (bc.held[dev] + bytes <= cap) {
-      bc.blocks.push_back({dev, p, bytes});
+      bc.blocks.push_back({dev, current_ctx_id(), p, bytes});
       bc.held[dev] += bytes;
       return;
     }
@@ -644,9 +652,10 @@ void handles_release(int dev) {
   {
     HandlePool &hp = handle_pool();
     std::lock_guard<std::mutex> lk(hp.m);
+    const unsigned long long ctx = current_ctx_id();
     for (size_t i = 0; i < hp.idle.size();) {
       if (hp.idle[i].first == dev) {
-        drop.push_back(hp.idle[i].second);
+        if (hp.idle[i].second.ctx == ctx) drop.push_back(hp.idle[i].second);
         hp.idle[i] = hp.idle.back();
         hp.idle.pop_back();
       } else {
@@ -659,17 +668,21 @@ void handles_release(int dev) {
 }  // namespace
 
 cudaError_t pdfs::handles_take(int dev, Handles *h) {
+  const unsigned long long ctx = current_ctx_id();
   {
     HandlePool &hp = handle_pool();
     std::lock_guard<std::mutex> lk(hp.m);
     for (size_t i = hp.idle.size(); i-- > 0;)
       if (hp.idle[i].first == dev) {
-        *h = hp.idle[i].second;
+        const Handles got = hp.idle[i].second;
         hp.idle[i] = hp.idle.back();
         hp.idle.pop_back();
+        if (got.ctx != ctx) continue;  // its context ended
+        *h = got;
         return cudaSuccess;
       }
   }
+  h->ctx = ctx;
   cudaError_t e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaHostAlloc(&h->pinned, kPinned, cudaHostAllocDefault);
   for (cudaEvent_t &ev : h->ev)
@@ -1115,6 +1128,10 @@ int pdfs::ctx_create(const pdfs_grid *g, const pdfs_opts *o_in, pdfs_ctx **out, 
 extern "C" void pdfs_ctx_destroy(pdfs_ctx *c) {
   if (!c) return;
   cudaSetDevice(c->dev);
+  if (c->hd.ctx != current_ctx_id()) {  // a reset ended the CUDA context: nothing of it is left
+    delete c;
+    return;
+  }
   // every block is idle before it goes back to the cache
   if (c->hd.st2) cudaStreamSynchronize(c->hd.st2);
   if (c->st) cudaStreamSynchronize(c->st);

@@ -21,6 +21,10 @@ static pthread_mutex_t mu = PTHREAD_MUTEX_INITIALIZER;
 static FILE *out;
 static uint64_t next_ptr = BASE, used, limit = 1ull << 38;
 static int next_id = 1, last_error, failed;
+/* the primary context: its id, and the first stream and address made in it */
+static unsigned long long ctx_id = 1;
+static int first_stream = 1;
+static uint64_t first_ptr = BASE;
 static struct { uint64_t p, n; } blocks[4096];
 static int nblocks;
 static struct { const void *fn; char name[256]; } kernels[4096];
@@ -34,6 +38,24 @@ __attribute__((constructor)) static void init(void) {
 #define SAY(...) (out ? (fprintf(out, __VA_ARGS__), fflush(out)) : 0)
 
 typedef struct { unsigned x, y, z; } dim3_;
+
+/* A stream or an address of a context that a reset ended: logged, and an error. */
+static int stale(const void *st, const void *p) {
+  const int s = (int)(intptr_t)st;
+  const uint64_t q = (uint64_t)(uintptr_t)p;
+  const int bad = (s && s < first_stream) || (q >= BASE && q < first_ptr);
+  if (bad) SAY("stale stream%d %llx\n", s, (unsigned long long)q);
+  return bad ? (last_error = 400) : 0; /* cudaErrorInvalidResourceHandle */
+}
+int cudaDeviceReset(void) {
+  SAY("reset\n");
+  ++ctx_id;
+  first_stream = next_id;
+  first_ptr = next_ptr;
+  used = 0;
+  nblocks = 0;
+  return 0;
+}
 
 /* launches */
 void **__cudaRegisterFatBinary(void *p) { return (void **)p; }
@@ -73,6 +95,7 @@ int __cudaPopCallConfiguration(dim3_ *g, dim3_ *b, size_t *s, void *st) {
 }
 int __cudaLaunchKernel(void *k, dim3_ g, dim3_ b, void **args, size_t s, void *st) {
   (void)b; (void)args; (void)s;
+  if (stale(st, NULL)) return 400;
   const char *name = "?", *f = getenv("FAKE_FAIL");
   pthread_mutex_lock(&mu);
   for (int i = 0; i < nkernels; ++i)
@@ -106,6 +129,7 @@ int cudaMalloc(void **p, size_t n) {
   return e;
 }
 int cudaFree(void *p) {
+  if (stale(NULL, p)) return 400;
   pthread_mutex_lock(&mu);
   for (int i = 0; i < nblocks; ++i)
     if (p && blocks[i].p == (uint64_t)(uintptr_t)p) {
@@ -144,7 +168,8 @@ int cudaMemcpy(void *d, const void *s, size_t n, int k) {
   return 0;
 }
 int cudaMemcpyAsync(void *d, const void *s, size_t n, int k, void *st) {
-  (void)d; (void)k;
+  (void)k;
+  if (stale(st, d) || stale(st, s)) return 400;
   const char *f = getenv("FAKE_COPIES"), *b = getenv("FAKE_COPY_BYTES");
   if (f && b && (size_t)atoll(b) == n && (uint64_t)(uintptr_t)s < BASE) {
     FILE *o = fopen(f, "ab");
@@ -165,7 +190,8 @@ int cudaMemset(void *d, int v, size_t n) {
   return 0;
 }
 int cudaMemsetAsync(void *d, int v, size_t n, void *st) {
-  (void)d; (void)v;
+  (void)v;
+  if (stale(st, d)) return 400;
   SAY("set %zu stream%d\n", n, (int)(intptr_t)st);
   return 0;
 }
@@ -177,10 +203,12 @@ int cudaStreamCreateWithFlags(void **s, unsigned f) {
   return 0;
 }
 int cudaStreamDestroy(void *s) {
+  if (stale(s, NULL)) return 400;
   SAY("destroy stream%d\n", (int)(intptr_t)s);
   return 0;
 }
 int cudaStreamSynchronize(void *s) {
+  if (stale(s, NULL)) return 400;
   SAY("wait stream%d\n", (int)(intptr_t)s);
   return 0;
 }
@@ -275,9 +303,18 @@ int cudaGetSymbolAddress(void **p, const void *s) {
   return 0;
 }
 static int encode_ok(void) { return 0; }
+static int get_current(void **c) {
+  *c = (void *)1;
+  return 0;
+}
+static int get_id(void *c, unsigned long long *id) {
+  (void)c;
+  *id = ctx_id;
+  return 0;
+}
 int cudaGetDriverEntryPointByVersion(const char *n, void **p, unsigned v, unsigned long long f, int *q) {
-  (void)n; (void)v; (void)f;
-  *p = (void *)encode_ok;
+  (void)v; (void)f;
+  *p = !strcmp(n, "cuCtxGetCurrent") ? (void *)get_current : !strcmp(n, "cuCtxGetId") ? (void *)get_id : (void *)encode_ok;
   if (q) *q = 0;
   return 0;
 }
